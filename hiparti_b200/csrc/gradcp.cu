@@ -5,6 +5,7 @@
 // of every factor is a per-mode MTTKRP of the residual; the Hadamard partials
 // are recomputed by the MTTKRP kernels rather than stored per nonzero.
 #include "kutil.cuh"
+#include "split.cuh"
 #include "tensor.cuh"
 #include "tma.cuh"
 
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(256) kruskal_values_kernel(KVArgs a)
 // mode-0 row keep that factor row in registers, so a nonzero gathers the
 // other modes' rows only (2 instead of 3 for a 3-mode tensor).  Each value is
 // written to its input position (the schedule's permutation).
-constexpr uint32_t kKsTile = 2048;  // records per CTA
+constexpr uint32_t kKsTile = 2048;  // records per CTA at most (split_for)
 #ifndef PTI_KS_U
 #define PTI_KS_U 3
 #endif
@@ -104,6 +105,7 @@ struct KSArgs {
     const float *mats[3];
     float *out;
     uint32_t *err;
+    uint32_t tile;  // records per CTA
 };
 
 template <int G, int NIN>
@@ -113,8 +115,8 @@ __global__ void __launch_bounds__(256) kruskal_sched_kernel(KSArgs a)
     __shared__ __align__(128) uint4 s_rec[kKsTile];
     __shared__ uint64_t mbar;
     const uint32_t tid = threadIdx.x;
-    const uint64_t z0 = (uint64_t)blockIdx.x * kKsTile;
-    const uint32_t n = (uint32_t)((a.nnz - z0) < kKsTile ? (a.nnz - z0) : kKsTile);
+    const uint64_t z0 = (uint64_t)blockIdx.x * a.tile;
+    const uint32_t n = (uint32_t)((a.nnz - z0) < a.tile ? (a.nnz - z0) : a.tile);
     if (tid == 0) {
         mbar_init(&mbar, 1);
         mbar_fence_init();
@@ -219,18 +221,26 @@ static int lanes_for(uint32_t R)
     return g;
 }
 
+template <int G, int NIN>
+static int launch_ks_g(KSArgs a, cudaStream_t s)
+{
+    static const uint64_t slots = cta_slots(kruskal_sched_kernel<G, NIN>, 256, 0);
+    a.tile = part_len(kKsTile, split_for((a.nnz + kKsTile - 1) / kKsTile, kKsTile, slots, 256 / G * kKsU));
+    kruskal_sched_kernel<G, NIN><<<(unsigned)((a.nnz + a.tile - 1) / a.tile), 256, 0, s>>>(a);
+    return 0;
+}
+
 template <int NIN>
-static int launch_ks(int G, const KSArgs &a, unsigned tiles, cudaStream_t s)
+static int launch_ks(int G, const KSArgs &a, cudaStream_t s)
 {
     switch (G) {
-        case 1: kruskal_sched_kernel<1, NIN><<<tiles, 256, 0, s>>>(a); break;
-        case 2: kruskal_sched_kernel<2, NIN><<<tiles, 256, 0, s>>>(a); break;
-        case 4: kruskal_sched_kernel<4, NIN><<<tiles, 256, 0, s>>>(a); break;
-        case 8: kruskal_sched_kernel<8, NIN><<<tiles, 256, 0, s>>>(a); break;
-        case 16: kruskal_sched_kernel<16, NIN><<<tiles, 256, 0, s>>>(a); break;
-        default: kruskal_sched_kernel<32, NIN><<<tiles, 256, 0, s>>>(a); break;
+        case 1: return launch_ks_g<1, NIN>(a, s);
+        case 2: return launch_ks_g<2, NIN>(a, s);
+        case 4: return launch_ks_g<4, NIN>(a, s);
+        case 8: return launch_ks_g<8, NIN>(a, s);
+        case 16: return launch_ks_g<16, NIN>(a, s);
+        default: return launch_ks_g<32, NIN>(a, s);
     }
-    return 0;
 }
 
 template <int NM>
@@ -291,8 +301,7 @@ int ptiB200KruskalValues(ptiB200Tensor *t, const float *const *dev_factors, ptiI
         for (uint32_t m = 0; m < t->nmodes; ++m) k.mats[m] = dev_factors[m];
         k.out = dev_out;
         k.err = err_word(t);
-        const unsigned tiles = (unsigned)((t->nnz + kKsTile - 1) / kKsTile);
-        PTI_TRY(t->nmodes == 3 ? launch_ks<2>(G, k, tiles, st) : launch_ks<1>(G, k, tiles, st));
+        PTI_TRY(t->nmodes == 3 ? launch_ks<2>(G, k, st) : launch_ks<1>(G, k, st));
         PTI_CUDA(cudaGetLastError(), mod);
         return 0;
     }

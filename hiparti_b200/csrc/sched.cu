@@ -25,12 +25,19 @@
 
 #include "kutil.cuh"
 #include "primitives.cuh"
+#include "split.cuh"
 #include "tensor.cuh"
 #include "tma.cuh"
 
 namespace pti {
 
-constexpr int kTile = 2048;        // nonzeros per CTA (COO kernel)
+
+// Nonzeros per CTA of the COO kernel at most.  Records of 8 words (4-D) with
+// FP32 rows take 1024, which fits a fourth CTA on an SM: 527 -> 507 us for the
+// four modes of a uniform 4-D tensor of 5M nonzeros at R = 32.  BF16 rows keep
+// 2048, as their walk feeds on the L1 that the fourth CTA's shared memory
+// would take (574 us, and 609 with 1024, for 5M Zipf nonzeros at R = 64).
+constexpr uint32_t coo_tile(int words, int cpl) { return cpl == 8 || words <= 4 ? 2048u : 8192u / words; }
 constexpr int kHiTile = kPlanTile; // nonzeros per CTA (HiCOO kernel)
 constexpr int kSchedThreads = 256;
 
@@ -55,6 +62,7 @@ struct SchedArgs {
     const uint4 *bquad;         // HiCOO 4-D: per block {output, operand 0, 1, 2} block coordinates
     const uint4 *recs;          // HiCOO: decoded records of the schedule (HicooModePlan::recs)
     const float *rvals;         // HiCOO 4-D: their values
+    uint32_t part;              // hicoo_rec_kernel: nonzeros per CTA, at most kHiTile
 };
 
 
@@ -627,6 +635,10 @@ struct RecSmem {
 // schedule already holds decoded (HicooModePlan::recs, in output-row order
 // within the tile): one bulk copy stages them (and the 4-D values), then the
 // thread groups walk contiguous slices (walk_rows).
+//
+// With few tiles each is cut into parts of a.part records, one CTA each
+// (split_for; blockIdx.y is the part): a part is contiguous and in row order
+// like its tile.
 template <int G, int CPL, int U, class FT, int NIN>
 __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kernel(SchedArgs a)
 {
@@ -639,8 +651,10 @@ __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kerne
     float *s_v3 = reinterpret_cast<float *>(sm + L::rval);
     float *s_slots = reinterpret_cast<float *>(sm + L::slots);
     const uint32_t tid = threadIdx.x;
-    const uint64_t z0 = (uint64_t)blockIdx.x * kHiTile;
-    const uint32_t n = (uint32_t)((a.nnz - z0) < (uint64_t)kHiTile ? (a.nnz - z0) : (uint64_t)kHiTile);
+    const uint32_t in_tile = blockIdx.y * a.part;  // < kHiTile: no part is empty in a full tile
+    const uint64_t z0 = (uint64_t)blockIdx.x * kHiTile + in_tile;
+    if (z0 >= a.nnz) return;
+    const uint32_t n = (uint32_t)min((uint64_t)min(a.part, kHiTile - in_tile), a.nnz - z0);
     if (tid == 0) {
         mbar_init(&mbar, 1);
         mbar_fence_init();
@@ -714,17 +728,18 @@ __global__ void build_records_kernel(RecBuildArgs r)
     }
 }
 
-// COO schedule: packed records sorted by output index; no sorting in the kernel.
+// COO schedule: packed records sorted by output index; no sorting in the
+// kernel.  A CTA takes `tile` records (launch_coo sizes it).
 template <int G, int CPL, int U, int MINB, class FT, int NIN>
-__global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArgs a, const uint32_t *recs)
+__global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArgs a, const uint32_t *recs, uint32_t tile)
 {
     constexpr int RW = Rec<NIN>::words;
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ uint64_t mbar;
     uint32_t *s_rec = reinterpret_cast<uint32_t *>(sm);
     const uint32_t tid = threadIdx.x;
-    const uint64_t z0 = (uint64_t)blockIdx.x * kTile;
-    const uint32_t n = (uint32_t)((a.nnz - z0) < (uint64_t)kTile ? (a.nnz - z0) : (uint64_t)kTile);
+    const uint64_t z0 = (uint64_t)blockIdx.x * tile;
+    const uint32_t n = (uint32_t)((a.nnz - z0) < (uint64_t)tile ? (a.nnz - z0) : (uint64_t)tile);
     if (tid == 0) {
         mbar_init(&mbar, 1);
         mbar_fence_init();
@@ -745,7 +760,7 @@ __global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArg
     }
     __shared__ uint32_t s_slot_row[kSchedThreads];
     __shared__ uint8_t s_slot_whole[kSchedThreads];
-    float *s_slots = reinterpret_cast<float *>(sm + (size_t)kTile * RW * 4);  // [groups][G][CPL]
+    float *s_slots = reinterpret_cast<float *>(sm + (size_t)tile * RW * 4);  // [groups][G][CPL]
     const uint32_t g = tid / G, lane = tid % G;
     constexpr uint32_t kGroups = kSchedThreads / G;
     const uint32_t per = ((n + kGroups - 1) / kGroups) | 1u;  // odd: groups start on different banks
@@ -1079,14 +1094,19 @@ int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals
 #endif
 
 template <int G, int CPL, int U, class FT, int NIN>
-static int launch_coo(const SchedArgs &a, const uint32_t *recs, unsigned ntiles, cudaStream_t s)
+static int launch_coo(const SchedArgs &a, const uint32_t *recs, cudaStream_t s)
 {
-    const size_t smem = (size_t)kTile * Rec<NIN>::words * 4 + (size_t)kSchedThreads * CPL * 4;
+    constexpr uint32_t RW = Rec<NIN>::words, kTile = coo_tile(RW, CPL);
+    constexpr size_t smem_max = (size_t)kTile * RW * 4 + (size_t)kSchedThreads * CPL * 4;
     constexpr int UU = NIN == 3 && U > 2 ? 2 : U;  // 4-D records hold more registers per nonzero
     auto k = coo_sched_kernel<G, CPL, UU, PTI_COO_MINB, FT, NIN>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max) != cudaSuccess)
         return PTIERR_CUDA_ERROR;
-    k<<<ntiles, kSchedThreads, smem, s>>>(a, recs);
+    static const uint64_t slots = cta_slots(k, kSchedThreads, smem_max);
+    const uint32_t split = split_for((a.nnz + kTile - 1) / kTile, kTile, slots, kSchedThreads / G * UU);
+    const uint32_t tile = part_len(kTile, split);
+    const size_t smem = (size_t)tile * RW * 4 + (size_t)kSchedThreads * CPL * 4;
+    k<<<(unsigned)((a.nnz + tile - 1) / tile), kSchedThreads, smem, s>>>(a, recs, tile);
     return 0;
 }
 
@@ -1111,27 +1131,36 @@ constexpr bool use_records()
 }
 
 template <int G, int CPL, class FT, int NIN>
-static int launch_hicoo(const SchedArgs &a, unsigned ntiles, cudaStream_t s)
+static int launch_hicoo(const SchedArgs &a0, unsigned ntiles, cudaStream_t s)
 {
     constexpr int U = NIN == 3 || CPL == 8 ? 2 : PTI_HICOO_U;  // nonzeros in flight per group
-    size_t smem;
-    void (*k)(SchedArgs);
-    if constexpr (use_records<FT, NIN>()) {
-        smem = RecSmem<NIN, CPL>::total;
-        if (sizeof(FT) == 2 && PTI_REC_BF16_CTAS > 0) {
-            // more dynamic shared memory than 1/(n+1) of the SM's 228 KB (with
-            // the static part and the 1 KB the runtime keeps per CTA)
-            const size_t cap = 233472 / (PTI_REC_BF16_CTAS + 1) - 1408 - 1024 + 16;
-            smem = smem > cap ? smem : cap;
-        }
-        k = hicoo_rec_kernel<G, CPL, U, FT, NIN>;
-    } else {
-        smem = HiSmem<NIN, CPL>::total;
-        k = hicoo_sched_kernel<G, CPL, U, FT, NIN>;
+    SchedArgs a = a0;
+    auto kr = hicoo_rec_kernel<G, CPL, U, FT, NIN>;
+    size_t rec_smem = RecSmem<NIN, CPL>::total;
+    if (sizeof(FT) == 2 && PTI_REC_BF16_CTAS > 0) {
+        // more dynamic shared memory than 1/(n+1) of the SM's 228 KB (with
+        // the static part and the 1 KB the runtime keeps per CTA)
+        const size_t cap = 233472 / (PTI_REC_BF16_CTAS + 1) - 1408 - 1024 + 16;
+        rec_smem = rec_smem > cap ? rec_smem : cap;
     }
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rec_smem) != cudaSuccess)
         return PTIERR_CUDA_ERROR;
-    k<<<ntiles, kSchedThreads, smem, s>>>(a);
+    static const uint64_t slots = cta_slots(kr, kSchedThreads, rec_smem);
+    a.part = part_len(kHiTile, split_for(ntiles, kHiTile, slots, kSchedThreads / G * U));
+    const unsigned parts = (kHiTile + a.part - 1) / a.part;
+    // whole tiles of 3-D FP32 runs are decoded in the kernel; parts of a tile
+    // come from the records, which need no block table
+    if constexpr (!use_records<FT, NIN>()) {
+        if (parts == 1) {
+            constexpr size_t smem = HiSmem<NIN, CPL>::total;
+            auto k = hicoo_sched_kernel<G, CPL, U, FT, NIN>;
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+                return PTIERR_CUDA_ERROR;
+            k<<<ntiles, kSchedThreads, smem, s>>>(a);
+            return 0;
+        }
+    }
+    kr<<<dim3(ntiles, parts), kSchedThreads, rec_smem, s>>>(a);
     return 0;
 }
 
@@ -1151,11 +1180,11 @@ static int launch_r(bool hicoo, bool wide, const SchedArgs &a, const uint32_t *r
                 if (R <= 64) return launch_hicoo<8, 8, FT, NIN>(a, ntiles, s);
                 return launch_hicoo<16, 8, FT, NIN>(a, ntiles, s);
             }
-            if (R <= 8) return launch_coo<1, 8, 2, FT, NIN>(a, recs, ntiles, s);
-            if (R <= 16) return launch_coo<2, 8, 2, FT, NIN>(a, recs, ntiles, s);
-            if (R <= 32) return launch_coo<4, 8, 2, FT, NIN>(a, recs, ntiles, s);
-            if (R <= 64) return launch_coo<8, 8, 2, FT, NIN>(a, recs, ntiles, s);
-            return launch_coo<16, 8, 2, FT, NIN>(a, recs, ntiles, s);
+            if (R <= 8) return launch_coo<1, 8, 2, FT, NIN>(a, recs, s);
+            if (R <= 16) return launch_coo<2, 8, 2, FT, NIN>(a, recs, s);
+            if (R <= 32) return launch_coo<4, 8, 2, FT, NIN>(a, recs, s);
+            if (R <= 64) return launch_coo<8, 8, 2, FT, NIN>(a, recs, s);
+            return launch_coo<16, 8, 2, FT, NIN>(a, recs, s);
         }
     }
     if (hicoo) {
@@ -1166,12 +1195,12 @@ static int launch_r(bool hicoo, bool wide, const SchedArgs &a, const uint32_t *r
         if (R <= 64) return launch_hicoo<16, 4, FT, NIN>(a, ntiles, s);
         return launch_hicoo<32, 4, FT, NIN>(a, ntiles, s);
     }
-    if (R <= 4) return launch_coo<1, 4, PTI_COO_U, FT, NIN>(a, recs, ntiles, s);
-    if (R <= 8) return launch_coo<2, 4, PTI_COO_U, FT, NIN>(a, recs, ntiles, s);
-    if (R <= 16) return launch_coo<4, 4, PTI_COO_U, FT, NIN>(a, recs, ntiles, s);
-    if (R <= 32) return launch_coo<8, 4, PTI_COO_U, FT, NIN>(a, recs, ntiles, s);
-    if (R <= 64) return launch_coo<16, 4, PTI_COO_U64, FT, NIN>(a, recs, ntiles, s);
-    return launch_coo<32, 4, 2, FT, NIN>(a, recs, ntiles, s);
+    if (R <= 4) return launch_coo<1, 4, PTI_COO_U, FT, NIN>(a, recs, s);
+    if (R <= 8) return launch_coo<2, 4, PTI_COO_U, FT, NIN>(a, recs, s);
+    if (R <= 16) return launch_coo<4, 4, PTI_COO_U, FT, NIN>(a, recs, s);
+    if (R <= 32) return launch_coo<8, 4, PTI_COO_U, FT, NIN>(a, recs, s);
+    if (R <= 64) return launch_coo<16, 4, PTI_COO_U64, FT, NIN>(a, recs, s);
+    return launch_coo<32, 4, 2, FT, NIN>(a, recs, s);
 }
 
 template <class FT>
@@ -1212,7 +1241,7 @@ int mttkrp_scheduled(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t
     a.out = out;
     a.err = err_word(t);
     const uint32_t *recs = nullptr;
-    unsigned ntiles;
+    unsigned ntiles = 0;
     if (t->hicoo) {
         const HicooModePlan &P = t->hicoo_plan[mode];
         ntiles = P.ntiles;
@@ -1240,7 +1269,6 @@ int mttkrp_scheduled(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t
         a.rvals = P.rvals.as<float>();
     } else {
         // records hold the operand modes in increasing order
-        ntiles = (unsigned)((t->nnz + kTile - 1) / kTile);
         CooModePlan &P = t->coo_plan[mode];
         recs = P.recs.as<uint32_t>();
         if (vals_override) {  // substituted values, brought into record order
