@@ -9,8 +9,7 @@
 //
 // Precision: factors are stored in FP32 (or, in mixed mode, additionally as a
 // BF16 copy that the MTTKRP gathers read); MTTKRP accumulates in FP32; Grams,
-// their Hadamard product, the Cholesky factor and inverse, the row solve and
-// the fit are FP64.  A Gram matrix that is not positive definite is inverted
+// their Hadamard product and its inverse, the row solve and the fit are FP64.  A Gram matrix that is not positive definite is inverted
 // by Gauss-Jordan elimination with partial pivoting (the reference falls back
 // to sgesv, src/matrix/matrix_solver.c:66-80); a singular one leaves the rows
 // unsolved, as sgesv does when it fails.
@@ -24,6 +23,7 @@
 #include <cmath>
 #include <limits>
 
+#include "als_dense.cuh"
 #include "checkpoint.cuh"
 #include "spd.cuh"
 #include "tensor.cuh"
@@ -32,128 +32,37 @@ namespace pti {
 
 constexpr int kMaxCpdRank = 128;
 
-// Gram accumulation: G += A^T A over rows [0, I).  If lambda is given the
-// rows are first divided column-wise by lambda (and written back); if bf16 is
-// given the (scaled) rows are also stored as BF16.  With round_bf16 the Gram
-// is formed from the BF16-rounded values -- the ones the next MTTKRPs gather --
-// so that an ALS step's right-hand side and normal matrix come from the same
-// factors (with FP32 Grams beside BF16 gathers the normal equations are
-// inconsistent, and inside an ALS swamp, where they are ill-conditioned, the
-// solve amplifies that until the iteration diverges).  Dynamic shared
-// memory: R*R doubles of accumulator + 32*R doubles of row tile.
-__global__ void gram_kernel(float *A, uint32_t I, uint32_t R, uint32_t stride, const float *lambda,
-                            __nv_bfloat16 *bf16, double *G, int round_bf16)
+// One CTA: W = (Hadamard_{k != mode} G_k)^{-1}, by symmetric sweeps
+// (sweep_inverse).  The Grams are read from their upper triangles.  zero_g
+// (R x R doubles) and zero_stats (zero_words ints), where given, are cleared on
+// the way: the accumulators that the steps after this one add into.  flag[0] = 0, or 1 if the matrix is not positive definite
+// (Gauss-Jordan with pivoting used), 2 if it is singular (W = identity: rows
+// left unsolved).  work holds 3*R*R doubles in global memory for that case.
+// The CTA of each instantiation covers its R with 4 to 16 elements a thread.
+template <int NTY, int PA, int PB>
+__global__ void __launch_bounds__(32 * NTY) gram_inverse_kernel(const double *G, uint32_t N, uint32_t R,
+                                                                uint32_t mode, double *W, double *work, int *flag,
+                                                                double *zero_g, int *zero_stats, uint32_t zero_words)
 {
-    extern __shared__ double sm[];
-    double *acc = sm;
-    double *tile = sm + (size_t)R * R;
+    __shared__ double s_row[2 * 32 * PB], s_rcp[2];
     const uint32_t RR = R * R;
-    for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) acc[e] = 0.0;
-    for (uint64_t r0 = (uint64_t)blockIdx.x * 32; r0 < I; r0 += (uint64_t)gridDim.x * 32) {
-        const uint32_t rows = (uint32_t)((I - r0) < 32 ? (I - r0) : 32);
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < 32 * stride; e += blockDim.x) {
-            const uint32_t r = e / stride, c = e % stride;
-            if (r >= rows) continue;
-            float *p = A + (r0 + r) * stride + c;
-            float v = *p;
-            if (c >= R) {
-                v = 0.f;
-                if (lambda) *p = 0.f;
-            } else if (lambda) {
-                v = v / lambda[c];
-                *p = v;
-            }
-            const __nv_bfloat16 h = __float2bfloat16_rn(v);
-            if (bf16) bf16[(r0 + r) * stride + c] = h;
-            if (c < R) tile[r * R + c] = round_bf16 ? (double)__bfloat162float(h) : (double)v;
-        }
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) {
-            const uint32_t p = e / R, q = e % R;
-            double s = 0.0;
-            for (uint32_t r = 0; r < rows; ++r) s += tile[r * R + p] * tile[r * R + q];
-            acc[e] += s;
-        }
-    }
-    __syncthreads();
-    for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) atomicAdd(G + e, acc[e]);
-}
-
-// One CTA: W = (Hadamard_{k != mode} G_k)^{-1}.  flag[0] = 1 if the Cholesky
-// factorisation failed (fallback used), 2 if the matrix was singular
-// (W = identity: rows left unsolved).  Ranks up to 32: the matrices sit in
-// shared memory and one warp factors them (spd_inverse).
-__global__ void gram_inverse_small_kernel(const double *G, uint32_t N, uint32_t R, uint32_t mode, double *W,
-                                          int *flag)
-{
-    __shared__ double sV[32 * 32], sL[32 * 32], sLi[32 * 32], sW[32 * 32];
-    const uint32_t RR = R * R;
-    for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) {
+    auto hadamard = [&](uint32_t i, uint32_t j) {
+        const uint32_t e = min(i, j) * R + max(i, j);
         double v = 1.0;
         for (uint32_t k = 1; k < N; ++k) v *= G[(size_t)((mode + k) % N) * RR + e];
-        sV[e] = v;
-    }
-    __syncthreads();
-    const int f = spd_inverse(sV, sL, sLi, sW, R);
-    for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) W[e] = sW[e];
-    if (threadIdx.x == 0) flag[0] = f;
-}
-
-// The same for ranks above 32; work holds 3*R*R doubles in global memory.
-__global__ void gram_inverse_kernel(const double *G, uint32_t N, uint32_t R, uint32_t mode, double *W,
-                                    double *work, int *flag)
-{
-    const uint32_t RR = R * R;
-    double *V = work, *L = work + RR, *Li = work + 2 * RR;
-    __shared__ int s_bad;
-    __shared__ double s_d;
-    for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) {
-        double v = 1.0;
-        for (uint32_t k = 1; k < N; ++k) v *= G[(size_t)((mode + k) % N) * RR + e];
-        V[e] = v;
-        L[e] = 0.0;
-        Li[e] = 0.0;
-    }
-    if (threadIdx.x == 0) s_bad = 0;
-    __syncthreads();
-    // Cholesky V = L L^T, column by column
-    for (uint32_t j = 0; j < R; ++j) {
-        if (threadIdx.x == 0) {
-            double d = V[j * R + j];
-            for (uint32_t k = 0; k < j; ++k) d -= L[j * R + k] * L[j * R + k];
-            if (!(d > 0.0)) s_bad = 1;
-            s_d = d > 0.0 ? sqrt(d) : 1.0;
-            L[j * R + j] = s_d;
-        }
-        __syncthreads();
-        if (s_bad) break;
-        for (uint32_t i = j + 1 + threadIdx.x; i < R; i += blockDim.x) {
-            double s = V[i * R + j];
-            for (uint32_t k = 0; k < j; ++k) s -= L[i * R + k] * L[j * R + k];
-            L[i * R + j] = s / s_d;
-        }
-        __syncthreads();
-    }
-    if (!s_bad) {
-        // Li = L^{-1}, one column per thread
-        for (uint32_t c = threadIdx.x; c < R; c += blockDim.x) {
-            for (uint32_t i = c; i < R; ++i) {
-                double s = (i == c) ? 1.0 : 0.0;
-                for (uint32_t k = c; k < i; ++k) s -= L[i * R + k] * Li[k * R + c];
-                Li[i * R + c] = s / L[i * R + i];
-            }
-        }
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) {
-            const uint32_t p = e / R, q = e % R;
-            double s = 0.0;
-            for (uint32_t k = max(p, q); k < R; ++k) s += Li[k * R + p] * Li[k * R + q];
-            W[e] = s;
-        }
+        return v;
+    };
+    if (zero_g)
+        for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) zero_g[e] = 0.0;
+    for (uint32_t e = threadIdx.x; e < zero_words; e += blockDim.x) zero_stats[e] = 0;
+    if (sweep_inverse<NTY, PA, PB>(
+            R, hadamard,
+            [&](uint32_t i, uint32_t j, double v) { W[i * R + j] = v; }, s_row, s_rcp)) {
         if (threadIdx.x == 0) flag[0] = 0;
         return;
     }
+    double *V = work, *L = work + RR, *Li = work + 2 * RR;
+    for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) V[e] = hadamard(e / R, e % R);
     // Gauss-Jordan with partial pivoting on [V | I]: L holds V, Li holds I.
     __syncthreads();
     for (uint32_t e = threadIdx.x; e < RR; e += blockDim.x) {
@@ -205,42 +114,16 @@ __global__ void gram_inverse_kernel(const double *G, uint32_t N, uint32_t R, uin
     if (threadIdx.x == 0) flag[0] = s_sing ? 2 : 1;
 }
 
-// A[i, :] = M[i, :] * W (W symmetric), FP64 accumulation; pad columns zeroed.
-// Accumulates per-column sums of squares (FP64) and maxima of the FP32 results.
-__global__ void solve_rows_kernel(const float *M, const double *W, uint32_t I, uint32_t R, uint32_t stride, float *A,
-                                  double *colsq, int *colmax)
+static void launch_gram_inverse(const double *G, uint32_t N, uint32_t R, uint32_t mode, double *W, double *work,
+                                int *flag, cudaStream_t s, double *zero_g = nullptr, int *zero_stats = nullptr,
+                                uint32_t zero_words = 0)
 {
-    extern __shared__ double sm[];
-    double *sW = sm;                         // R*R
-    double *s_sq = sm + (size_t)R * R;       // R
-    int *s_mx = reinterpret_cast<int *>(s_sq + R);  // R
-    for (uint32_t e = threadIdx.x; e < R * R; e += blockDim.x) sW[e] = W[e];
-    for (uint32_t c = threadIdx.x; c < R; c += blockDim.x) {
-        s_sq[c] = 0.0;
-        s_mx[c] = 0;  // bits of +0.0f
-    }
-    __syncthreads();
-    const uint64_t total = (uint64_t)I * stride;
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t i = e / stride;
-        const uint32_t c = (uint32_t)(e % stride);
-        if (c >= R) {
-            A[e] = 0.f;
-            continue;
-        }
-        const float *m = M + i * stride;
-        double s = 0.0;
-        for (uint32_t k = 0; k < R; ++k) s += (double)m[k] * sW[k * R + c];
-        const float v = (float)s;
-        A[e] = v;
-        atomicAdd(&s_sq[c], (double)v * (double)v);
-        if (v > 0.f) atomicMax(&s_mx[c], __float_as_int(v));
-    }
-    __syncthreads();
-    for (uint32_t c = threadIdx.x; c < R; c += blockDim.x) {
-        atomicAdd(&colsq[c], s_sq[c]);
-        atomicMax(&colmax[c], s_mx[c]);
-    }
+    auto go = [&](auto k, unsigned threads) {
+        k<<<1, threads, 0, s>>>(G, N, R, mode, W, work, flag, zero_g, zero_stats, zero_words);
+    };
+    if (R <= 32) go(gram_inverse_kernel<8, 4, 1>, 256);
+    else if (R <= 64) go(gram_inverse_kernel<16, 4, 2>, 512);
+    else go(gram_inverse_kernel<32, 4, 4>, 1024);
 }
 
 // lambda from the column statistics: iteration 0 -> 2-norm
@@ -282,6 +165,7 @@ __global__ void sumsq_kernel(const float *v, uint64_t n, double *out)
     if ((threadIdx.x & 31) == 0) atomicAdd(out, s);
 }
 
+// Grams from their upper triangles:
 // fit = 1 - sqrt(normX2 + |lambda^T (Hadamard_k G_k) lambda| - 2 inner) / sqrt(normX2)
 // (src/ktensor/ktensor.c:77-99: the square root is skipped if the residual is
 // not positive).
@@ -291,9 +175,10 @@ __global__ void fit_kernel(const double *G, uint32_t N, uint32_t R, const float 
     __shared__ double s_part[32];
     double s = 0.0;
     for (uint32_t e = threadIdx.x; e < R * R; e += blockDim.x) {
+        const uint32_t i = e / R, j = e % R;
         double v = 1.0;
-        for (uint32_t k = 0; k < N; ++k) v *= G[(size_t)k * R * R + e];
-        s += v * (double)lambda[e / R] * (double)lambda[e % R];
+        for (uint32_t k = 0; k < N; ++k) v *= G[(size_t)k * R * R + min(i, j) * R + max(i, j)];
+        s += v * (double)lambda[i] * (double)lambda[j];
     }
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = s;
@@ -323,17 +208,18 @@ __global__ void colsq_kernel(const float *A, uint32_t I, uint32_t R, uint32_t st
     for (uint32_t c = threadIdx.x; c < R; c += blockDim.x) atomicAdd(&colsq[c], s_sq[c]);
 }
 
-// A[:, c] /= norm_c ; lambda_c *= norm_c (src/matrix/matrix.c:556-572)
+// A[:, c] /= norm_c ; lambda_c *= norm_c (src/matrix/matrix.c:556-572), the
+// squared norm of column c at colsq[c * step] (a Gram's diagonal: step R + 1)
 __global__ void final_scale_kernel(float *A, uint32_t I, uint32_t R, uint32_t stride, const double *colsq,
-                                   float *lambda, int update_lambda)
+                                   float *lambda, int update_lambda, uint32_t step)
 {
     const uint64_t total = (uint64_t)I * stride;
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t c = (uint32_t)(e % stride);
-        if (c < R) A[e] = A[e] / (float)sqrt(colsq[c]);
+        if (c < R) A[e] = A[e] / (float)sqrt(colsq[(size_t)c * step]);
     }
     if (update_lambda && blockIdx.x == 0)
-        for (uint32_t c = threadIdx.x; c < R; c += blockDim.x) lambda[c] *= (float)sqrt(colsq[c]);
+        for (uint32_t c = threadIdx.x; c < R; c += blockDim.x) lambda[c] *= (float)sqrt(colsq[(size_t)c * step]);
 }
 
 // ---------------------------------------------------------------------------
@@ -419,23 +305,26 @@ int cpd_device(ptiB200Tensor *t, float *const *A, uint32_t stride, float *lambda
     CkptWriter writer;
     if (opt.ckpt_path) PTI_TRY(writer.init(opt.ckpt_path, N, t->ndims.data(), t->nnz, R, opt.niters));
 
-    const size_t gram_smem = (size_t)(RR + 32 * R) * 8;
-    const size_t solve_smem = (size_t)RR * 8 + (size_t)R * 12;
-    PTI_CUDA(cudaFuncSetAttribute(gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem), mod);
-    PTI_CUDA(cudaFuncSetAttribute(solve_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem), mod);
     const unsigned sms = (unsigned)sm_count();
     auto rows_grid = [&](uint64_t items, unsigned per) {
         return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((items + per - 1) / per, sms * 4ull));
     };
 
-    // Grams of every factor (cpd.c:65-72) and their BF16 copies; with
-    // round_bf16 the Grams are of the BF16-rounded factors (gram_kernel)
+    // With round_bf16 a Gram is formed from the BF16-rounded values -- the ones
+    // the next MTTKRPs gather -- so that an ALS step's right-hand side and
+    // normal matrix come from the same factors (with FP32 Grams beside BF16
+    // gathers the normal equations are inconsistent, and inside an ALS swamp,
+    // where they are ill-conditioned, the solve amplifies that until the
+    // iteration diverges).
+    auto gram_args = [&](uint32_t m, int scale, int round_bf16) {
+        return GramArgs{A[m], t->ndims[m], R, stride, scale, colsq, colmax, lambda,
+                        mixed ? Ab[m].as<__nv_bfloat16>() : nullptr, round_bf16, G.as<double>() + (size_t)m * RR};
+    };
+    // Grams of every factor (cpd.c:65-72) and their BF16 copies
     auto all_grams = [&](int round_bf16) -> int {
         PTI_CUDA(cudaMemsetAsync(G.ptr, 0, (size_t)N * RR * 8, s), mod);
         for (uint32_t m = 0; m < N; ++m)
-            gram_kernel<<<rows_grid(t->ndims[m], 32), 256, gram_smem, s>>>(
-                A[m], t->ndims[m], R, stride, nullptr, mixed ? Ab[m].as<__nv_bfloat16>() : nullptr,
-                G.as<double>() + (size_t)m * RR, round_bf16);
+            PTI_CUDA(launch_gram(gram_args(m, 0, round_bf16), s), mod);
         return 0;
     };
     const uint32_t it_first = have_ckpt ? st.iters : 0;
@@ -488,25 +377,16 @@ int cpd_device(ptiB200Tensor *t, float *const *A, uint32_t stride, float *lambda
             for (uint32_t i = 0; i < N; ++i) order[i] = (m + i) % N;
             PTI_CUDA(cudaEventRecord(ev.g, s), mod);
             PTI_CUDA(cudaStreamWaitEvent(side, ev.g, 0), mod);
-            if (R <= 32)
-                gram_inverse_small_kernel<<<1, 256, 0, side>>>(G.as<double>(), N, R, m, W.as<double>(), flag);
-            else
-                gram_inverse_kernel<<<1, 256, 0, side>>>(G.as<double>(), N, R, m, W.as<double>(), work.as<double>(),
-                                                         flag);
+            launch_gram_inverse(G.as<double>(), N, R, m, W.as<double>(), work.as<double>(), flag, side,
+                                G.as<double>() + (size_t)m * RR, stats.as<int>(), 3 * R);
             PTI_CUDA(cudaGetLastError(), mod);
             PTI_CUDA(cudaEventRecord(ev.w, side), mod);
             PTI_TRY(mttkrp_device(t, fptr.data(), use_bf16 ? PTI_B200_BF16 : PTI_B200_F32, R, stride, order.data(), m,
                                   M.as<float>(), s));
             PTI_CUDA(cudaStreamWaitEvent(s, ev.w, 0), mod);
-            PTI_CUDA(cudaMemsetAsync(stats.ptr, 0, (size_t)R * 12, s), mod);
-            solve_rows_kernel<<<rows_grid((uint64_t)t->ndims[m] * stride, 256), 256, solve_smem, s>>>(
-                M.as<float>(), W.as<double>(), t->ndims[m], R, stride, A[m], colsq, colmax);
-            lambda_kernel<<<1, 128, 0, s>>>(colsq, colmax, R, it == 0, lambda);
-            PTI_CUDA(cudaMemsetAsync(G.as<double>() + (size_t)m * RR, 0, (size_t)RR * 8, s), mod);
-            gram_kernel<<<rows_grid(t->ndims[m], 32), 256, gram_smem, s>>>(
-                A[m], t->ndims[m], R, stride, lambda, mixed ? Ab[m].as<__nv_bfloat16>() : nullptr,
-                G.as<double>() + (size_t)m * RR, use_bf16);
-            PTI_CUDA(cudaGetLastError(), mod);
+            PTI_CUDA(launch_solve_rows(M.as<float>(), W.as<double>(), t->ndims[m], R, stride, A[m], colsq, colmax, s),
+                     mod);
+            PTI_CUDA(launch_gram(gram_args(m, it == 0 ? 1 : 2, use_bf16), s), mod);
         }
         const uint32_t last = N - 1;
         PTI_CUDA(cudaMemsetAsync(inner, 0, 8, s), mod);
@@ -531,13 +411,18 @@ int cpd_device(ptiB200Tensor *t, float *const *A, uint32_t stride, float *lambda
     if (opt.m_last && it > 0 && t->ndims[N - 1])
         PTI_CUDA(cudaMemcpyAsync(opt.m_last, M.ptr, (size_t)t->ndims[N - 1] * stride * 4, cudaMemcpyDeviceToDevice, s),
                  mod);
-    // GetFinalLambda (matrix.c:556-572)
+    // GetFinalLambda (matrix.c:556-572).  The squared column norms are the
+    // Grams' diagonals, unless those are of the BF16-rounded factors.
     for (uint32_t m = 0; m < N; ++m) {
-        PTI_CUDA(cudaMemsetAsync(colsq, 0, (size_t)R * 8, s), mod);
-        colsq_kernel<<<rows_grid((uint64_t)t->ndims[m] * stride, 256), 256, R * 8, s>>>(A[m], t->ndims[m], R, stride,
-                                                                                        colsq);
-        final_scale_kernel<<<rows_grid((uint64_t)t->ndims[m] * stride, 256), 256, 0, s>>>(A[m], t->ndims[m], R,
-                                                                                          stride, colsq, lambda, 1);
+        const double *sq = G.as<double>() + (size_t)m * RR;
+        if (grams_bf16) {
+            sq = colsq;
+            PTI_CUDA(cudaMemsetAsync(colsq, 0, (size_t)R * 8, s), mod);
+            colsq_kernel<<<rows_grid((uint64_t)t->ndims[m] * stride, 256), 256, R * 8, s>>>(A[m], t->ndims[m], R,
+                                                                                            stride, colsq);
+        }
+        final_scale_kernel<<<rows_grid((uint64_t)t->ndims[m] * stride, 256), 256, 0, s>>>(
+            A[m], t->ndims[m], R, stride, sq, lambda, 1, grams_bf16 ? 1 : R + 1);
     }
     PTI_CUDA(cudaGetLastError(), mod);
     res.fits.resize(it);
@@ -826,25 +711,16 @@ int normals(uint32_t mode, uint32_t nmodes, Mat **aTa, Mat *rhs, const char *mod
         PTI_CUDA(flag.alloc(64, s), mod);
         // the inverse kernels multiply the Grams of every mode but `mode`; with
         // the one product matrix as "mode 0 of two", that is the product itself
-        if (R <= 32) {
-            gram_inverse_small_kernel<<<1, 256, 0, s>>>(out64.as<double>(), 2, R, 1, W.as<double>(), flag.as<int>());
-        } else {
-            PTI_CUDA(work.alloc(padded((size_t)3 * R * R * 8), s), mod);
-            gram_inverse_kernel<<<1, 256, 0, s>>>(out64.as<double>(), 2, R, 1, W.as<double>(), work.as<double>(),
-                                                  flag.as<int>());
-        }
+        PTI_CUDA(work.alloc(padded((size_t)3 * R * R * 8), s), mod);
+        launch_gram_inverse(out64.as<double>(), 2, R, 1, W.as<double>(), work.as<double>(), flag.as<int>(), s);
         PTI_CUDA(Min.alloc(padded((size_t)I * stride * 4), s), mod);
         PTI_CUDA(Aout.alloc(padded((size_t)I * stride * 4), s), mod);
         PTI_CUDA(stats.alloc(padded((size_t)R * 12 + 64), s), mod);
         PTI_CUDA(cudaMemsetAsync(stats.ptr, 0, (size_t)R * 12, s), mod);
         PTI_CUDA(cudaMemcpyAsync(Min.ptr, rhs->values, (size_t)I * stride * 4, cudaMemcpyHostToDevice, s), mod);
-        const size_t solve_smem = (size_t)R * R * 8 + (size_t)R * 12;
-        PTI_CUDA(cudaFuncSetAttribute(solve_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem),
+        PTI_CUDA(launch_solve_rows(Min.as<float>(), W.as<double>(), I, R, stride, Aout.as<float>(), stats.as<double>(),
+                                   reinterpret_cast<int *>(stats.as<double>() + R), s),
                  mod);
-        solve_rows_kernel<<<rows_grid_for((uint64_t)I * stride), 256, solve_smem, s>>>(
-            Min.as<float>(), W.as<double>(), I, R, stride, Aout.as<float>(), stats.as<double>(),
-            reinterpret_cast<int *>(stats.as<double>() + R));
-        PTI_CUDA(cudaGetLastError(), mod);
         int hflag = 0;
         PTI_CUDA(cudaMemcpyAsync(&hflag, flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, s), mod);
         PTI_CUDA(cudaStreamSynchronize(s), mod);
@@ -912,7 +788,7 @@ int final_lambda(uint32_t rank, uint32_t nmodes, Mat **mats, float *lambda, cons
                                                                                            stride, colsq.as<double>());
         }
         final_scale_kernel<<<rows_grid_for((uint64_t)std::max<uint32_t>(I, 1) * stride), 256, 0, s>>>(
-            dA.as<float>(), I, rank, stride, colsq.as<double>(), lam.as<float>(), 1);
+            dA.as<float>(), I, rank, stride, colsq.as<double>(), lam.as<float>(), 1, 1);
         PTI_CUDA(cudaGetLastError(), mod);
         if (I) PTI_CUDA(cudaMemcpyAsync(A->values, dA.ptr, (size_t)I * stride * 4, cudaMemcpyDeviceToHost, s), mod);
         PTI_CUDA(cudaStreamSynchronize(s), mod);
