@@ -383,19 +383,6 @@ __device__ double block_sum(double x, double *red)
     return red[kBThreads / 32];
 }
 
-// Accumulates G += v v^T for one row held one column per lane (lanes >= R hold
-// 0): lane c keeps row c of G in g[].
-__device__ __forceinline__ void gram_row(double (&g)[kBMaxRank], float v, uint32_t R)
-{
-#pragma unroll
-    for (int k = 0; k < kBMaxRank; ++k) {
-        if (k < (int)R) {
-            const float vk = __shfl_sync(0xffffffffu, v, k);
-            g[k] = fma((double)v, (double)vk, g[k]);
-        }
-    }
-}
-
 // The mode-m ALS step of one tensor (one CTA).  With gram_bf16 (the
 // iterations whose MTTKRPs gather BF16 factors) the new Gram is formed from
 // the BF16-rounded factor, the values those gathers read, so that the next
@@ -423,11 +410,6 @@ __device__ void dense_task(const BatchTensor *__restrict__ gt, uint32_t b, uint3
 
     for (uint32_t e = tid; e < RR; e += kBThreads) {
         V[e] = __ldcg(G + (size_t)ma * RR + e) * __ldcg(G + (size_t)mb * RR + e);
-        Gs[e] = 0.0;
-    }
-    if (tid < kBMaxRank) {
-        s_colsq[tid] = 0.0;
-        s_colmax[tid] = 0;
     }
     __syncthreads();
     spd_inverse(V, Lm, Li, W, R);
@@ -501,17 +483,33 @@ __device__ void dense_task(const BatchTensor *__restrict__ gt, uint32_t b, uint3
                 }
             }
         }
+        // the lanes of a column, then the warps (an FP64 atomic in shared
+        // memory is a compare-and-swap loop): partials in the row tiles, which
+        // pass 2 fills later
+        double *psq = reinterpret_cast<double *>(sm + DenseSmem::rows);
+        float *pmx = reinterpret_cast<float *>(psq + kWarps * kBMaxRank);
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            if (nt >= (int)NT) break;
+        for (int j = 0; j < 8; ++j) {
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const uint32_t col = 8 * nt + 2 * t4 + i;
-                if (col < R) {
-                    atomicAdd(&s_colsq[col], csq[2 * nt + i]);
-                    atomicMax(&s_colmax[col], __float_as_int(cmx[2 * nt + i]));
-                }
+            for (int o = 4; o < 32; o <<= 1) {
+                csq[j] += __shfl_xor_sync(0xffffffffu, csq[j], o);
+                cmx[j] = fmaxf(cmx[j], __shfl_xor_sync(0xffffffffu, cmx[j], o));
             }
+            if (g8 == 0) {
+                psq[warp * kBMaxRank + 8 * (j >> 1) + 2 * t4 + (j & 1)] = csq[j];
+                pmx[warp * kBMaxRank + 8 * (j >> 1) + 2 * t4 + (j & 1)] = cmx[j];
+            }
+        }
+        __syncthreads();
+        if (tid < R) {
+            double sq = 0.0;
+            float mx = 0.f;
+            for (uint32_t w = 0; w < kWarps; ++w) {
+                sq += psq[w * kBMaxRank + tid];
+                mx = fmaxf(mx, pmx[w * kBMaxRank + tid]);
+            }
+            s_colsq[tid] = sq;
+            s_colmax[tid] = __float_as_int(mx);
         }
     }
     __syncthreads();
@@ -572,22 +570,45 @@ __device__ void dense_task(const BatchTensor *__restrict__ gt, uint32_t b, uint3
             }
             __syncwarp();
         }
-        // add the warp's tiles into the Gram: tile (p, q) holds G[8p + g][8q + 2t + i]
-        int j = 0;
+        // add the warps' tiles, half of the warps to the other half at a time
+        // through the matrices that the inverse no longer needs
+        double *part = reinterpret_cast<double *>(sm + DenseSmem::V);
+        for (uint32_t h = kWarps / 2; h > 0; h >>= 1) {
+            __syncthreads();
+            double *slot = part + (size_t)(warp < h ? warp : warp - h) * 20 * 32 + lane;
+            if (warp >= h && warp < 2 * h) {
 #pragma unroll
-        for (int pt = 0; pt < 4; ++pt)
-#pragma unroll
-            for (int qt = pt; qt < 4; ++qt, ++j) {
-                if (qt >= (int)NT) continue;
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const uint32_t r = 8 * pt + g8, c = 8 * qt + 2 * t4 + i;
-                    if (r < R && c < R) {
-                        atomicAdd(&Gs[r * R + c], gacc[j][i]);
-                        if (pt != qt) atomicAdd(&Gs[c * R + r], gacc[j][i]);
-                    }
+                for (int j = 0; j < 10; ++j) {
+                    slot[(2 * j) * 32] = gacc[j][0];
+                    slot[(2 * j + 1) * 32] = gacc[j][1];
                 }
             }
+            __syncthreads();
+            if (warp < h) {
+#pragma unroll
+                for (int j = 0; j < 10; ++j) {
+                    gacc[j][0] += slot[(2 * j) * 32];
+                    gacc[j][1] += slot[(2 * j + 1) * 32];
+                }
+            }
+        }
+        // tile (p, q) holds G[8p + g][8q + 2t + i]
+        if (warp == 0) {
+            int j = 0;
+#pragma unroll
+            for (int pt = 0; pt < 4; ++pt)
+#pragma unroll
+                for (int qt = pt; qt < 4; ++qt, ++j) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const uint32_t r = 8 * pt + g8, c = 8 * qt + 2 * t4 + i;
+                        if (r < R && c < R) {
+                            Gs[r * R + c] = gacc[j][i];
+                            if (pt != qt) Gs[c * R + r] = gacc[j][i];
+                        }
+                    }
+                }
+        }
     }
     // zero the next mode's MTTKRP output (its tiles wait for this step)
     {
@@ -672,35 +693,77 @@ __global__ void bump_kernel(uint32_t *iter) { *iter += 1; }
 
 // Grams of the current factors and their BF16 copies; one CTA per (tensor,
 // mode).  With round_bf16 the Grams are of the BF16-rounded factors (the
-// values the BF16 iterations gather, see dense_task).
+// values the BF16 iterations gather, see dense_task).  Tensor-core tiles as in
+// dense_task: both operands of a tile product are the same fragment, so a lane
+// loads each element it needs itself.  (Rows broadcast column by column
+// through shuffles took 1.18 ms for 128 tensors of up to 5,000 rows a mode;
+// this takes 0.08.)
 __global__ void __launch_bounds__(kBThreads) batch_init_kernel(const BatchTensor *tens, int mixed, int round_bf16)
 {
-    __shared__ double Gs[kBMaxRank * kBMaxRank];
+    __shared__ double part[kBThreads / 64][20][32];
     const BatchTensor *gt = tens + blockIdx.x / 3;
     const uint32_t m = blockIdx.x % 3;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
     const uint32_t R = gt->R, stride = gt->stride, RR = R * R, I = gt->dims[m];
     const float *A = gt->A[m];
     __nv_bfloat16 *Ab = gt->Ab[m];
-    for (uint32_t e = tid; e < RR; e += kBThreads) Gs[e] = 0.0;
-    __syncthreads();
-    double g[kBMaxRank];
+    double acc[10][2];
 #pragma unroll
-    for (int k = 0; k < kBMaxRank; ++k) g[k] = 0.0;
-    for (uint32_t i = warp; i < I; i += kBThreads / 32) {
-        const size_t e = (size_t)i * stride + lane;
-        const float v = lane < R ? A[e] : 0.f;
-        const __nv_bfloat16 h = __float2bfloat16_rn(v);
-        if (mixed && lane < stride) Ab[e] = h;
-        gram_row(g, round_bf16 ? __bfloat162float(h) : v, R);
-    }
-    if (lane < R) {
+    for (int j = 0; j < 10; ++j) acc[j][0] = acc[j][1] = 0.0;
+    for (uint32_t i0 = warp * 16; i0 < I; i0 += kBThreads / 32 * 16) {
+        float v[4][4];
 #pragma unroll
-        for (int k = 0; k < kBMaxRank; ++k)
-            if (k < (int)R) atomicAdd(&Gs[lane * R + k], g[k]);
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const uint32_t row = i0 + 4 * k + t4, col = 8 * n + g8;
+                v[k][n] = row < I && col < R ? A[(size_t)row * stride + col] : 0.f;
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            double fr[4];
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const uint32_t row = i0 + 4 * k + t4, col = 8 * n + g8;
+                const __nv_bfloat16 h = __float2bfloat16_rn(v[k][n]);
+                if (mixed && row < I && col < stride) Ab[(size_t)row * stride + col] = h;
+                fr[n] = round_bf16 ? (double)__bfloat162float(h) : (double)v[k][n];
+            }
+            int j = 0;
+#pragma unroll
+            for (int pt = 0; pt < 4; ++pt)
+#pragma unroll
+                for (int qt = pt; qt < 4; ++qt, ++j) dmma(acc[j][0], acc[j][1], fr[pt], fr[qt]);
+        }
     }
-    __syncthreads();
-    for (uint32_t e = tid; e < RR; e += kBThreads) gt->G[(size_t)m * RR + e] = Gs[e];
+    for (uint32_t h = kBThreads / 64; h > 0; h >>= 1) {
+        __syncthreads();
+        if (warp >= h && warp < 2 * h) {
+#pragma unroll
+            for (int j = 0; j < 20; ++j) part[warp - h][j][lane] = acc[j / 2][j & 1];
+        }
+        __syncthreads();
+        if (warp < h) {
+#pragma unroll
+            for (int j = 0; j < 20; ++j) acc[j / 2][j & 1] += part[warp][j][lane];
+        }
+    }
+    if (warp == 0) {
+        double *G = gt->G + (size_t)m * RR;
+        int j = 0;
+#pragma unroll
+        for (int pt = 0; pt < 4; ++pt)
+#pragma unroll
+            for (int qt = pt; qt < 4; ++qt, ++j)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t r = 8 * pt + g8, c = 8 * qt + 2 * t4 + i;
+                    if (r < R && c < R) {
+                        G[r * R + c] = acc[j][i];
+                        if (pt != qt) G[c * R + r] = acc[j][i];
+                    }
+                }
+    }
 }
 
 // ||X||^2 of every tensor; one CTA per tensor.
@@ -715,31 +778,27 @@ __global__ void batch_norm_kernel(const float *const *vals, const uint64_t *nnz,
     if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
-// Final lambda (src/matrix/matrix.c:556-572): every column of every factor is
-// normalised and lambda takes the norms; one CTA per tensor.
-__global__ void __launch_bounds__(kBThreads) batch_final_kernel(const BatchTensor *tens)
+// Column sums of squares of the FP32 factors into the Grams' diagonals, for a
+// last iteration whose Grams are of the BF16-rounded factors.
+__global__ void __launch_bounds__(kBThreads) batch_colsq_kernel(const BatchTensor *tens)
 {
-    __shared__ double s_sq[kBMaxRank];
-    const BatchTensor *gt = tens + blockIdx.x;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t R = gt->R, stride = gt->stride;
-    for (uint32_t m = 0; m < 3; ++m) {
-        float *A = gt->A[m];
-        const uint32_t I = gt->dims[m];
-        if (tid < kBMaxRank) s_sq[tid] = 0.0;
-        __syncthreads();
-        double sq = 0.0;
-        for (uint32_t i = warp; i < I; i += kBThreads / 32)
-            if (lane < R) {
-                const double v = A[(size_t)i * stride + lane];
-                sq += v * v;
-            }
-        if (lane < R) atomicAdd(&s_sq[lane], sq);
-        __syncthreads();
-        for (uint32_t i = warp; i < I; i += kBThreads / 32)
-            if (lane < R) A[(size_t)i * stride + lane] /= (float)sqrt(s_sq[lane]);
-        if (tid < R) gt->lambda[tid] *= (float)sqrt(s_sq[tid]);
-        __syncthreads();
+    __shared__ double part[kBThreads / 32][kBMaxRank];
+    const BatchTensor *gt = tens + blockIdx.x / 3;
+    const uint32_t m = blockIdx.x % 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t R = gt->R, stride = gt->stride, I = gt->dims[m];
+    const float *A = gt->A[m];
+    double sq = 0.0;
+#pragma unroll 8
+    for (uint32_t i = warp; i < I; i += kBThreads / 32) {
+        const double v = lane < R ? A[(size_t)i * stride + lane] : 0.f;
+        sq += v * v;
+    }
+    part[warp][lane] = sq;
+    __syncthreads();
+    if (threadIdx.x < R) {
+        double s = 0.0;
+        for (int w = 0; w < kBThreads / 32; ++w) s += part[w][threadIdx.x];
+        gt->G[((size_t)m * R + threadIdx.x) * R + threadIdx.x] = s;
     }
 }
 
@@ -749,17 +808,51 @@ struct CopyItem {
     uint64_t n;  // floats
 };
 
-// One CTA per item; 16-byte copies where both ends allow them.
-__global__ void batch_copy_kernel(const CopyItem *items)
+// The result (src/matrix/matrix.c:556-572): the columns of every factor divided
+// by their norms -- the square roots of the Grams' diagonals -- on their way to
+// the caller, and lambda multiplied by them.  items: the 3 factors of every
+// tensor, then every lambda.  blockIdx.x: factor, blockIdx.y: part of its rows.
+// (One CTA per tensor, its modes and the norms one after another, then a copy:
+// 1.48 + 0.09 ms for 128 tensors; this takes 0.08.)
+constexpr uint32_t kOutParts = 8;
+__global__ void __launch_bounds__(kBThreads) batch_out_kernel(const BatchTensor *tens, const CopyItem *items,
+                                                              uint32_t B)
+{
+    __shared__ float s_norm[kBMaxRank];
+    const uint32_t b = blockIdx.x / 3, m = blockIdx.x % 3, tid = threadIdx.x;
+    const BatchTensor *gt = tens + b;
+    const uint32_t R = gt->R, stride = gt->stride;
+    if (tid < kBMaxRank) s_norm[tid] = tid < R ? (float)sqrt(gt->G[((size_t)m * R + tid) * R + tid]) : 1.f;
+    if (m == 0 && blockIdx.y == 0 && tid < R) {
+        float l = gt->lambda[tid];
+        for (uint32_t k = 0; k < 3; ++k) l *= (float)sqrt(gt->G[((size_t)k * R + tid) * R + tid]);
+        items[3 * B + b].dst[tid] = l;
+    }
+    __syncthreads();
+    const CopyItem c = items[blockIdx.x];  // rows of `stride` floats, 16-byte aligned at both ends
+    const float4 *src = reinterpret_cast<const float4 *>(c.src);
+    float4 *dst = reinterpret_cast<float4 *>(c.dst);
+    const uint32_t q = stride / 4;
+    for (uint64_t e = (uint64_t)blockIdx.y * kBThreads + tid; e < c.n / 4; e += (uint64_t)kOutParts * kBThreads) {
+        const uint32_t col = (uint32_t)(e % q) * 4;
+        float4 v = src[e];
+        v.x /= s_norm[col];
+        v.y /= s_norm[col + 1];
+        v.z /= s_norm[col + 2];
+        v.w /= s_norm[col + 3];
+        dst[e] = v;
+    }
+}
+
+// blockIdx.x: item, blockIdx.y: part of it.  The items are factors: multiples
+// of 8 floats, 16-byte aligned at both ends.
+__global__ void __launch_bounds__(kBThreads) batch_copy_kernel(const CopyItem *items)
 {
     const CopyItem c = items[blockIdx.x];
-    if (((uintptr_t)c.src | (uintptr_t)c.dst) % 16 == 0 && c.n % 4 == 0) {
-        const float4 *s = reinterpret_cast<const float4 *>(c.src);
-        float4 *d = reinterpret_cast<float4 *>(c.dst);
-        for (uint64_t i = threadIdx.x; i < c.n / 4; i += blockDim.x) d[i] = s[i];
-    } else {
-        for (uint64_t i = threadIdx.x; i < c.n; i += blockDim.x) c.dst[i] = c.src[i];
-    }
+    const float4 *s = reinterpret_cast<const float4 *>(c.src);
+    float4 *d = reinterpret_cast<float4 *>(c.dst);
+    for (uint64_t i = (uint64_t)blockIdx.y * kBThreads + threadIdx.x; i < c.n / 4; i += (uint64_t)kOutParts * kBThreads)
+        d[i] = s[i];
 }
 
 // Fills the factor arena with values in [0.1, 1.1) from a hash (used to time
@@ -1287,14 +1380,13 @@ int ptiB200BatchCpdAls(ptiB200Batch *bt, ptiIndex niters, int precision, ptiInde
     PTI_CUDA(bt->copies.alloc(padded(items.size() * sizeof(CopyItem)), s), kMod);
     PTI_CUDA(cudaMemcpyAsync(bt->copies.ptr, items.data(), 3 * (size_t)B * sizeof(CopyItem), cudaMemcpyHostToDevice,
                              s), kMod);
-    batch_copy_kernel<<<3 * B, 256, 0, s>>>(bt->copies.as<CopyItem>());
+    batch_copy_kernel<<<dim3(3 * B, kOutParts), kBThreads, 0, s>>>(bt->copies.as<CopyItem>());
     PTI_TRY(batch_init_factors(bt, mixed, mixed && niters > fp32_sweeps));
     DevBuf dfits;
     PTI_CUDA(dfits.alloc(padded((size_t)B * niters * 8), s), kMod);
     float ms = 0.f;
     PTI_TRY(batch_iterate(bt, niters, mixed, fp32_sweeps, bt->cpl, dfits.as<double>(), &ms));
-    batch_final_kernel<<<B, kBThreads, 0, s>>>(bt->tens.as<BatchTensor>());
-    // factors and lambda out: arena -> caller's arrays
+    // factors and lambda out, normalised: arena -> caller's arrays
     std::vector<CopyItem> outs(4 * (size_t)B);
     for (uint32_t b = 0; b < B; ++b) {
         for (uint32_t m = 0; m < 3; ++m)
@@ -1305,7 +1397,9 @@ int ptiB200BatchCpdAls(ptiB200Batch *bt, ptiIndex niters, int precision, ptiInde
     PTI_CUDA(out_items.alloc(padded(outs.size() * sizeof(CopyItem)), s), kMod);
     PTI_CUDA(cudaMemcpyAsync(out_items.ptr, outs.data(), outs.size() * sizeof(CopyItem), cudaMemcpyHostToDevice, s),
              kMod);
-    batch_copy_kernel<<<4 * B, 256, 0, s>>>(out_items.as<CopyItem>());
+    if (mixed && fp32_sweeps == 0)  // the last Grams are of the BF16-rounded factors
+        batch_colsq_kernel<<<3 * B, kBThreads, 0, s>>>(bt->tens.as<BatchTensor>());
+    batch_out_kernel<<<dim3(3 * B, kOutParts), kBThreads, 0, s>>>(bt->tens.as<BatchTensor>(), out_items.as<CopyItem>(), B);
     PTI_CUDA(cudaGetLastError(), kMod);
     if (fits) PTI_CUDA(cudaMemcpyAsync(fits, dfits.ptr, (size_t)B * niters * 8, cudaMemcpyDeviceToHost, s), kMod);
     PTI_CUDA(cudaStreamSynchronize(s), kMod);
