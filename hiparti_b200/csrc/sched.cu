@@ -682,52 +682,6 @@ __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kerne
     walk_rows<G, CPL, U, FT, NIN>(s_rec, s_v3, n, j0, j1, g, lane, a, s_slots, s_slot_row, s_slot_whole);
 }
 
-// Decodes a HiCOO schedule into records (HicooModePlan::recs): the nonzero at
-// schedule position j lies in block tile_block[j / kHiTile] + lblk[j] of the
-// schedule's block order.  Operands in increasing mode order.
-struct RecBuildArgs {
-    uint64_t n, nb;
-    uint32_t nin, sb;
-    const uint16_t *lblk;
-    const uint32_t *tile_block;
-    const uint32_t *out_bind;
-    const uint8_t *out_eind;
-    uint32_t out_dim;
-    const uint32_t *in_bind[3];
-    const uint8_t *in_eind[3];
-    uint32_t in_dim[3];
-    const float *vals;
-    uint4 *recs;
-    float *rvals;
-    uint32_t *err;
-};
-
-__global__ void build_records_kernel(RecBuildArgs r)
-{
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < r.n; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t b0 = (uint64_t)r.tile_block[j / kHiTile] + r.lblk[j];
-        const bool ok_b = b0 < r.nb;
-        const uint64_t b = ok_b ? b0 : 0;
-        const uint64_t o = ((uint64_t)r.out_bind[b] << r.sb) + r.out_eind[j];
-        const bool ok_o = ok_b && o < r.out_dim;
-        uint32_t row[3] = {0u, 0u, 0u};
-        bool ok_in = true;
-        for (uint32_t k = 0; k < r.nin; ++k) {
-            const uint64_t rk = ((uint64_t)r.in_bind[k][b] << r.sb) + r.in_eind[k][j];
-            ok_in = ok_in && rk < r.in_dim[k];
-            row[k] = (uint32_t)rk;
-        }
-        if (!ok_in) row[0] = row[1] = row[2] = 0u;
-        const float v = ok_o && ok_in ? r.vals[j] : 0.f;
-        uint4 rec = make_uint4(ok_o ? (uint32_t)o : kNoRow, row[0], row[1], row[2]);
-        if (r.nin == 1) rec.z = __float_as_uint(v);
-        if (r.nin == 2) rec.w = __float_as_uint(v);
-        if (r.nin == 3) r.rvals[j] = v;
-        r.recs[j] = rec;
-        if (!(ok_o && ok_in)) atomicOr(r.err, 1u);
-    }
-}
-
 // COO schedule: packed records sorted by output index; no sorting in the
 // kernel.  A CTA takes `tile` records (launch_coo sizes it).
 template <int G, int CPL, int U, int MINB, class FT, int NIN>
@@ -772,21 +726,12 @@ __global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArg
 // ---------------------------------------------------------------------------
 // Schedule construction
 // ---------------------------------------------------------------------------
-__global__ void iota_keys_kernel(const uint32_t *src, uint64_t n, uint64_t *keys, uint32_t *vals)
+__global__ void iota_keys_kernel(const uint32_t *src, uint64_t n, uint32_t *keys, uint32_t *vals)
 {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         keys[i] = src[i];
         vals[i] = (uint32_t)i;
     }
-}
-
-// 4-D schedules: each block's coordinates as one record {output mode,
-// operand modes in increasing order}.
-__global__ void pack_bquad_kernel(const uint32_t *bo, const uint32_t *b0, const uint32_t *b1, const uint32_t *b2,
-                                  uint64_t nb, uint4 *q)
-{
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += (uint64_t)gridDim.x * blockDim.x)
-        q[i] = make_uint4(bo[i], b0[i], b1[i], b2[i]);
 }
 
 // COO packed records in sorted order: {out index, operand indices (modes in
@@ -810,77 +755,196 @@ __global__ void pack_records_kernel(PackArgs pa, const uint32_t *perm, uint64_t 
     }
 }
 
-__global__ void block_of_nnz_kernel(const uint64_t *bptr, uint64_t nb, uint32_t *blk)
-{
-    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += (uint64_t)gridDim.x * blockDim.x)
-        for (uint64_t z = bptr[b]; z < bptr[b + 1]; ++z) blk[z] = (uint32_t)b;
-}
+// The schedule order of one tile of kHiTile nonzeros, by one CTA: the blocks
+// in their new order (bperm) with their nonzeros behind one another, then
+// stably by output row.  Writes for each position the nonzero there (order)
+// and its block, counted from the tile's first (lblk).
+//
+// The blocks are ascending in their output coordinate, so a tile spans few
+// rows: a stable radix sort by 8-bit digits of the row, counted from the tile's
+// first, takes one pass for most tiles and at most four.  (A bitonic sort of
+// 64-bit {row, position} pairs, fed by passes that spelt out every nonzero's
+// block, took 0.63 ms a mode for 10M Zipf nonzeros; this takes 0.20.)
+struct TileOrderArgs {
+    uint64_t nnz, nb;
+    uint32_t sb;
+    const uint32_t *tile_block;
+    const uint64_t *nbptr;   // first nonzero of each block in the new order
+    const uint32_t *bperm;   // new order -> block
+    const uint32_t *out_bind;
+    const uint64_t *bptr;
+    const uint8_t *out_eind;
+    uint32_t *order;
+    uint16_t *lblk;
+};
 
-__global__ void permuted_blocks_kernel(const uint32_t *perm, uint64_t nb, const uint64_t *bptr, uint32_t *size,
-                                       uint32_t *inv)
+__global__ void __launch_bounds__(kSortThreads) tile_order_kernel(TileOrderArgs t)
 {
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nb; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t b = perm[j];
-        size[j] = (uint32_t)(bptr[b + 1] - bptr[b]);
-        inv[b] = (uint32_t)j;
-    }
-}
-
-// Position of every nonzero in block order (blocks in their new order, the
-// nonzeros of a block in their stored order): order[pos] = z.
-__global__ void block_order_kernel(const uint32_t *blk, const uint32_t *inv, const uint64_t *bptr,
-                                   const uint64_t *nbptr, uint64_t n, uint32_t *order)
-{
-    for (uint64_t z = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; z < n; z += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t b = blk[z];
-        order[nbptr[inv[b]] + (z - bptr[b])] = (uint32_t)z;
-    }
-}
-
-// One CTA per tile of the block order: stable sort of the tile's nonzeros by
-// output row (a bitonic sort of (row, position) pairs in shared memory).
-__global__ void __launch_bounds__(256) tile_sort_kernel(const uint32_t *order, uint64_t n, const uint32_t *blk,
-                                                        const uint32_t *bout, const uint8_t *eout, uint32_t sb,
-                                                        uint32_t *sorted)
-{
-    constexpr uint32_t T = kHiTile;
-    static_assert((T & (T - 1)) == 0 && T <= 4096, "tile must be a power of two of at most 4096");
-    __shared__ uint64_t key[T];
+    constexpr uint32_t T = kHiTile, PER = T / kSortThreads;
+    static_assert(T == 32 * PER * kSortWarps && T <= 2048, "shared memory");
+    __shared__ uint32_t s_key[2][T], s_z[T], s_cnt[kSortWarps][256], s_warp[32], s_min, s_max;
+    __shared__ uint16_t s_pos[2][T], s_l[T];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t z0 = (uint64_t)blockIdx.x * T;
-    const uint32_t cnt = (uint32_t)((n - z0) < T ? (n - z0) : T);
-    for (uint32_t i = threadIdx.x; i < T; i += blockDim.x) {
-        if (i < cnt) {
-            const uint32_t z = order[z0 + i];
-            const uint64_t row = ((uint64_t)bout[blk[z]] << sb) + eout[z];
-            key[i] = (row << 12) | i;
-        } else {
-            key[i] = ~0ull;  // padding sorts last
-        }
+    const uint32_t cnt = (uint32_t)((t.nnz - z0) < T ? (t.nnz - z0) : T);
+    const uint32_t b0 = t.tile_block[blockIdx.x];
+    const uint32_t nblk = (uint32_t)min((uint64_t)min(t.tile_block[blockIdx.x + 1] - b0 + 1, T + 1), t.nb - b0);
+    // each position's block: the number of blocks that start up to it
+    for (uint32_t i = tid; i < T; i += kSortThreads) s_key[1][i] = 0;
+    if (tid == 0) {
+        s_min = 0xFFFFFFFFu;
+        s_max = 0;
     }
     __syncthreads();
-    for (uint32_t k = 2; k <= T; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < T; i += blockDim.x) {
-                const uint32_t ixj = i ^ j;
-                if (ixj > i) {
-                    const uint64_t x = key[i], y = key[ixj];
-                    if ((x > y) == ((i & k) == 0)) {
-                        key[i] = y;
-                        key[ixj] = x;
-                    }
-                }
-            }
-            __syncthreads();
+    for (uint32_t i = tid; i < nblk; i += kSortThreads) {
+        const uint64_t st = t.nbptr[b0 + i];
+        if (st < z0 + cnt) s_key[1][st > z0 ? (uint32_t)(st - z0) : 0u] = 1u;
+    }
+    __syncthreads();
+    uint32_t row[PER], sum = 0, total, lo = 0xFFFFFFFFu, hi = 0;
+#pragma unroll
+    for (uint32_t p = 0; p < PER; ++p) sum += s_key[1][tid * PER + p];
+    uint32_t run = block_exclusive_scan<uint32_t>(sum, s_warp, total);
+#pragma unroll
+    for (uint32_t p = 0; p < PER; ++p) {
+        const uint32_t pos = tid * PER + p;
+        run += s_key[1][pos];
+        row[p] = 0xFFFFFFFFu;
+        if (pos < cnt) {
+            const uint32_t i = run - 1, b = t.bperm[b0 + i];
+            const uint32_t z = (uint32_t)(t.bptr[b] + (z0 + pos - t.nbptr[b0 + i]));
+            s_z[pos] = z;
+            s_l[pos] = (uint16_t)i;
+            // (a coordinate beyond 32 bits is out of range: behind every row)
+            const uint64_t o = ((uint64_t)t.out_bind[b] << t.sb) + t.out_eind[z];
+            row[p] = o < 0xFFFFFFFFull ? (uint32_t)o : 0xFFFFFFFFu;
+            lo = min(lo, row[p]);
+            hi = max(hi, row[p]);
         }
-    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) sorted[z0 + i] = order[z0 + (uint32_t)(key[i] & 4095u)];
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) {
+        atomicMin(&s_min, lo);
+        atomicMax(&s_max, hi);
+    }
+    __syncthreads();
+    const uint32_t first = s_min, range = s_max - first;
+#pragma unroll
+    for (uint32_t p = 0; p < PER; ++p) {
+        const uint32_t pos = tid * PER + p;
+        s_key[0][pos] = pos < cnt ? row[p] - first : 0xFFFFFFFFu;  // past the end: behind every nonzero
+        s_pos[0][pos] = (uint16_t)pos;
+    }
+    uint32_t cur = 0;
+    for (uint32_t shift = 0; shift < 32 && range >> shift; shift += 8, cur ^= 1) {
+#pragma unroll
+        for (int w = 0; w < kSortWarps; ++w) s_cnt[w][tid] = 0;
+        __syncthreads();
+        uint32_t key[PER], rank[PER];
+#pragma unroll
+        for (uint32_t r = 0; r < PER; ++r) {
+            key[r] = s_key[cur][warp * (32 * PER) + 32 * r + lane];
+            rank[r] = warp_digit_rank(key[r] >> shift & 0xFFu, s_cnt[warp]);
+        }
+        __syncthreads();
+        digit_starts(s_cnt, s_warp);
+        __syncthreads();
+#pragma unroll
+        for (uint32_t r = 0; r < PER; ++r) {
+            const uint32_t to = s_cnt[warp][key[r] >> shift & 0xFFu] + rank[r];
+            s_key[cur ^ 1][to] = key[r];
+            s_pos[cur ^ 1][to] = s_pos[cur][warp * (32 * PER) + 32 * r + lane];
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    for (uint32_t j = tid; j < cnt; j += kSortThreads) {
+        const uint32_t pos = s_pos[cur][j];
+        t.order[z0 + j] = s_z[pos];
+        t.lblk[z0 + j] = s_l[pos];
+    }
 }
 
-// Block of the nonzero at position j, counted from the first block of its tile.
-__global__ void local_block_kernel(const uint32_t *order, uint64_t n, const uint32_t *blk, const uint32_t *inv,
-                                   const uint32_t *tile_block, uint16_t *lblk)
+// The schedule's arrays, gathered in its order in two passes: the blocks'
+// coordinates, then everything of a nonzero, its decoded record included
+// (HicooModePlan::recs; the nonzero at position j lies in block
+// tile_block[j / kHiTile] + lblk[j]).  Operands in increasing mode order.
+struct PlanGatherArgs {
+    uint64_t n, nb;
+    uint32_t nmodes, mode, sb;
+    uint32_t dims[kMaxModes];
+    const uint32_t *bperm, *order, *tile_block;
+    const uint16_t *lblk;
+    const uint32_t *binds_in[kMaxModes];
+    const uint8_t *einds_in[kMaxModes];
+    const float *vals_in;
+    uint32_t *binds[kMaxModes];
+    uint8_t *einds[kMaxModes];
+    float *vals;
+    uint4 *bquad;   // 4-D: {output, operands}
+    uint4 *recs;
+    float *rvals;   // 4-D
+    uint32_t *err;
+};
+
+__global__ void __launch_bounds__(256) plan_blocks_kernel(PlanGatherArgs g)
 {
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x)
-        lblk[j] = (uint16_t)(inv[blk[order[j]]] - tile_block[j / kHiTile]);
+    for (uint64_t j = (uint64_t)blockIdx.x * 256 + threadIdx.x; j < g.nb; j += (uint64_t)gridDim.x * 256) {
+        const uint32_t b = g.bperm[j];
+        uint32_t c[kMaxModes], q[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int k = 0; k < kMaxModes; ++k)
+            if (k < (int)g.nmodes) g.binds[k][j] = c[k] = g.binds_in[k][b];
+        if (g.bquad) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q[k == (int)g.mode ? 0 : k < (int)g.mode ? k + 1 : k] = c[k];
+            g.bquad[j] = make_uint4(q[0], q[1], q[2], q[3]);
+        }
+    }
+}
+
+template <int N>
+__global__ void __launch_bounds__(256) plan_nonzeros_kernel(PlanGatherArgs g)
+{
+    for (uint64_t j = (uint64_t)blockIdx.x * 256 + threadIdx.x; j < g.n; j += (uint64_t)gridDim.x * 256) {
+        const uint32_t z = g.order[j];
+        const uint64_t b0 = (uint64_t)g.tile_block[j / kHiTile] + g.lblk[j];
+        const float val = g.vals_in[z];
+        const bool ok_b = b0 < g.nb;
+        const uint64_t b = ok_b ? b0 : 0;
+        uint32_t row[3] = {0u, 0u, 0u}, out = 0;
+        bool ok_in = true, ok_o = ok_b;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const uint8_t e = g.einds_in[k][z];
+            g.einds[k][j] = e;
+            const uint64_t c = ((uint64_t)g.binds[k][b] << g.sb) + e;
+            const bool ok = c < g.dims[k];
+            if (k == (int)g.mode) {
+                out = (uint32_t)c;
+                ok_o = ok_o && ok;
+            } else {
+                ok_in = ok_in && ok;
+                const int i = k < (int)g.mode ? k : k - 1;
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+                    if (x == i) row[x] = (uint32_t)c;
+            }
+        }
+        g.vals[j] = val;
+        if (!ok_in) row[0] = row[1] = row[2] = 0u;
+        const float v = ok_o && ok_in ? val : 0.f;
+        uint4 rec = make_uint4(ok_o ? out : kNoRow, row[0], row[1], row[2]);
+        if (N == 2) rec.z = __float_as_uint(v);
+        if (N == 3) rec.w = __float_as_uint(v);
+        if (N == 4) g.rvals[j] = v;
+        g.recs[j] = rec;
+        if (!(ok_o && ok_in)) atomicOr(g.err, 1u);
+    }
 }
 
 template <class T>
@@ -900,9 +964,14 @@ __global__ void tile_block_kernel_t(const uint64_t *bptr, uint64_t nb, uint32_t 
     }
 }
 
-struct SizeIn {
-    const uint32_t *p;
-    __device__ uint64_t operator()(uint64_t i) const { return p[i]; }
+struct SizeIn {  // nonzeros of a block of the new order
+    const uint32_t *perm;
+    const uint64_t *bptr;
+    __device__ uint64_t operator()(uint64_t i) const
+    {
+        const uint32_t b = perm[i];
+        return bptr[b + 1] - bptr[b];
+    }
 };
 struct BptrOut {
     uint64_t *p;
@@ -934,11 +1003,11 @@ int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals
         if (P.ready) return 0;
         PTI_CHECK(N <= 4, PTIERR_VALUE_ERROR, mod, "COO schedules cover orders up to 4");
         DevBuf keys, perm;
-        RadixScratch rs;
-        PTI_CUDA(keys.alloc(padded(n * 8), s), mod);
+        RadixScratchT<uint32_t> rs;
+        PTI_CUDA(keys.alloc(padded(n * 4), s), mod);
         PTI_CUDA(perm.alloc(padded(n * 4), s), mod);
         PTI_TRY(rs.alloc(n, s));
-        iota_keys_kernel<<<grid_n(n), 256, 0, s>>>(t->inds[mode].as<uint32_t>(), n, keys.as<uint64_t>(),
+        iota_keys_kernel<<<grid_n(n), 256, 0, s>>>(t->inds[mode].as<uint32_t>(), n, keys.as<uint32_t>(),
                                                    perm.as<uint32_t>());
         PTI_TRY(radix_sort_pairs(keys, perm, n, (int)bits_for_count(t->ndims[mode]), rs, s));
         const int RW = N <= 3 ? 4 : 8;
@@ -957,121 +1026,96 @@ int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals
         return 0;
     }
     HicooModePlan &P = t->hicoo_plan[mode];
-    if (P.ready) return 0;
+    if (P.ready || N > 4) return 0;  // a record holds three operand rows; other orders take the direct kernel
     const uint64_t nb = t->nb;
     PTI_CHECK(t->sb <= 8, PTIERR_VALUE_ERROR, mod, "sb_bits must be <= 8");
     // 1. blocks by output-mode block coordinate (stable)
-    DevBuf bkeys, bperm, inv, bsize, nbptr;
+    DevBuf bkeys, bperm, nbptr, order;
     {
-        RadixScratch rs;
-        PTI_CUDA(bkeys.alloc(padded(nb * 8), s), mod);
+        RadixScratchT<uint32_t> rs;
+        PTI_CUDA(bkeys.alloc(padded(nb * 4), s), mod);
         PTI_CUDA(bperm.alloc(padded(nb * 4), s), mod);
         PTI_TRY(rs.alloc(nb, s));
-        iota_keys_kernel<<<grid_n(nb), 256, 0, s>>>(t->binds[mode].as<uint32_t>(), nb, bkeys.as<uint64_t>(),
+        iota_keys_kernel<<<grid_n(nb), 256, 0, s>>>(t->binds[mode].as<uint32_t>(), nb, bkeys.as<uint32_t>(),
                                                     bperm.as<uint32_t>());
         const uint64_t brows = ((uint64_t)t->ndims[mode] + ((uint64_t)1 << t->sb) - 1) >> t->sb;
-        PTI_TRY(radix_sort_pairs(bkeys, bperm, nb, (int)bits_for_count(brows + 1), rs, s));
+        PTI_TRY(radix_sort_pairs(bkeys, bperm, nb, (int)std::min(32u, bits_for_count(brows + 1)), rs, s));
     }
     bkeys.reset();
-    PTI_CUDA(inv.alloc(padded(nb * 4), s), mod);
-    PTI_CUDA(bsize.alloc(padded(nb * 4), s), mod);
-    permuted_blocks_kernel<<<grid_n(nb), 256, 0, s>>>(bperm.as<uint32_t>(), nb, t->bptr.as<uint64_t>(),
-                                                      bsize.as<uint32_t>(), inv.as<uint32_t>());
     PTI_CUDA(nbptr.alloc(padded((nb + 1) * 8), s), mod);
     {
         DevBuf tmp;
         PTI_CUDA(tmp.alloc(padded(scan_tmp_elems<uint64_t>(nb) * 8), s), mod);
-        PTI_TRY((exclusive_scan<uint64_t>(SizeIn{bsize.as<uint32_t>()}, BptrOut{nbptr.as<uint64_t>()}, nb,
-                                          tmp.as<uint64_t>(), nullptr, s)));
+        PTI_TRY((exclusive_scan<uint64_t>(SizeIn{bperm.as<uint32_t>(), t->bptr.as<uint64_t>()},
+                                          BptrOut{nbptr.as<uint64_t>()}, nb, tmp.as<uint64_t>(), nullptr, s)));
         PTI_CUDA(cudaMemcpyAsync(nbptr.as<uint64_t>() + nb, tmp.as<uint64_t>() + (nb + kScanTile - 1) / kScanTile,
                                  8, cudaMemcpyDeviceToDevice, s), mod);
     }
-    bsize.reset();
     P.nb = nb;
     P.ntiles = (uint32_t)((n + kHiTile - 1) / kHiTile);
     PTI_CUDA(P.tile_block.alloc(padded(((size_t)P.ntiles + 1) * 4), s), mod);
     tile_block_kernel_t<<<grid_n(nb), 256, 0, s>>>(nbptr.as<uint64_t>(), nb, P.ntiles, kHiTile,
                                                    P.tile_block.as<uint32_t>());
-    {
-        // 2. nonzeros in block order (blocks in their new order), then 3. inside
-        // each tile of that order by output row
-        DevBuf blk, border, order;
-        PTI_CUDA(blk.alloc(padded(n * 4), s), mod);
-        block_of_nnz_kernel<<<grid_n(nb), 256, 0, s>>>(t->bptr.as<uint64_t>(), nb, blk.as<uint32_t>());
-        PTI_CUDA(border.alloc(padded(n * 4), s), mod);
-        block_order_kernel<<<grid_n(n), 256, 0, s>>>(blk.as<uint32_t>(), inv.as<uint32_t>(), t->bptr.as<uint64_t>(),
-                                                     nbptr.as<uint64_t>(), n, border.as<uint32_t>());
-        PTI_CUDA(order.alloc(padded(n * 4), s), mod);
-        tile_sort_kernel<<<P.ntiles, 256, 0, s>>>(border.as<uint32_t>(), n, blk.as<uint32_t>(),
-                                                  t->binds[mode].as<uint32_t>(), t->einds[mode].as<uint8_t>(), t->sb,
-                                                  order.as<uint32_t>());
-        border.reset();
-        // 4. everything up to here read only bptr and the output mode's arrays;
-        // the gathers below read every array, each after its own arrival
-        // (with `arr`), in the order the arrays arrive: the output mode's,
-        // the values, then the other modes
-        PTI_CUDA(P.lblk.alloc(padded(n * 2), s), mod);
-        local_block_kernel<<<grid_n(n), 256, 0, s>>>(order.as<uint32_t>(), n, blk.as<uint32_t>(), inv.as<uint32_t>(),
-                                                     P.tile_block.as<uint32_t>(), P.lblk.as<uint16_t>());
-        auto wait = [&](cudaEvent_t ev) -> int {
-            if (ev) PTI_CUDA(cudaStreamWaitEvent(s, ev, 0), mod);
-            return 0;
-        };
-        auto gather_mode = [&](uint32_t k) -> int {
-            if (arr) PTI_TRY(wait(arr->mode[k]));
-            PTI_CUDA(P.binds[k].alloc(padded(nb * 4), s), mod);
-            gather_kernel<uint32_t><<<grid_n(nb), 256, 0, s>>>(t->binds[k].as<uint32_t>(), bperm.as<uint32_t>(), nb,
-                                                               P.binds[k].as<uint32_t>());
-            PTI_CUDA(P.einds[k].alloc(padded(n), s), mod);
-            gather_kernel<uint8_t><<<grid_n(n), 256, 0, s>>>(t->einds[k].as<uint8_t>(), order.as<uint32_t>(), n,
-                                                             P.einds[k].as<uint8_t>());
-            return 0;
-        };
-        PTI_TRY(gather_mode(mode));
-        if (arr) PTI_TRY(wait(arr->vals));
-        PTI_CUDA(P.vals.alloc(padded(n * 4), s), mod);
-        gather_kernel<float><<<grid_n(n), 256, 0, s>>>(t->vals.as<float>(), order.as<uint32_t>(), n,
-                                                       P.vals.as<float>());
+    // 2. nonzeros in block order (blocks in their new order), inside each tile
+    // of that order by output row
+    PTI_CUDA(order.alloc(padded(n * 4), s), mod);
+    PTI_CUDA(P.lblk.alloc(padded(n * 2), s), mod);
+    TileOrderArgs ta{};
+    ta.nnz = n;
+    ta.nb = nb;
+    ta.sb = t->sb;
+    ta.tile_block = P.tile_block.as<uint32_t>();
+    ta.nbptr = nbptr.as<uint64_t>();
+    ta.bperm = bperm.as<uint32_t>();
+    ta.out_bind = t->binds[mode].as<uint32_t>();
+    ta.bptr = t->bptr.as<uint64_t>();
+    ta.out_eind = t->einds[mode].as<uint8_t>();
+    ta.order = order.as<uint32_t>();
+    ta.lblk = P.lblk.as<uint16_t>();
+    tile_order_kernel<<<P.ntiles, kSortThreads, 0, s>>>(ta);
+    // 3. everything up to here read only bptr and the output mode's arrays;
+    // the gathers read every array, after its arrival (with `arr`)
+    if (arr) {
+        if (arr->vals) PTI_CUDA(cudaStreamWaitEvent(s, arr->vals, 0), mod);
         for (uint32_t k = 0; k < N; ++k)
-            if (k != mode) PTI_TRY(gather_mode(k));
-        bperm.reset();
-        if (N == 4) {
-            uint32_t o[3], c = 0;
-            for (uint32_t k = 0; k < N; ++k)
-                if (k != mode) o[c++] = k;
-            PTI_CUDA(P.bquad.alloc(padded(nb * 16), s), mod);
-            pack_bquad_kernel<<<grid_n(nb), 256, 0, s>>>(P.binds[mode].as<uint32_t>(), P.binds[o[0]].as<uint32_t>(),
-                                                         P.binds[o[1]].as<uint32_t>(), P.binds[o[2]].as<uint32_t>(),
-                                                         nb, P.bquad.as<uint4>());
-        }
-        // 5. the decoded records the MTTKRP kernel stages
-        PTI_TRY(ensure_err_word(t, s));
-        PTI_CUDA(P.recs.alloc(padded(n * 16), s), mod);
-        if (N == 4) PTI_CUDA(P.rvals.alloc(padded(n * 4), s), mod);
-        RecBuildArgs ra{};
-        ra.n = n;
-        ra.nb = nb;
-        ra.nin = N - 1;
-        ra.sb = t->sb;
-        ra.lblk = P.lblk.as<uint16_t>();
-        ra.tile_block = P.tile_block.as<uint32_t>();
-        ra.out_bind = P.binds[mode].as<uint32_t>();
-        ra.out_eind = P.einds[mode].as<uint8_t>();
-        ra.out_dim = t->ndims[mode];
-        for (uint32_t k = 0, i = 0; k < N; ++k)
-            if (k != mode) {
-                ra.in_bind[i] = P.binds[k].as<uint32_t>();
-                ra.in_eind[i] = P.einds[k].as<uint8_t>();
-                ra.in_dim[i] = t->ndims[k];
-                ++i;
-            }
-        ra.vals = P.vals.as<float>();
-        ra.recs = P.recs.as<uint4>();
-        ra.rvals = N == 4 ? P.rvals.as<float>() : nullptr;
-        ra.err = err_word(t);
-        build_records_kernel<<<grid_n(n), 256, 0, s>>>(ra);
+            if (arr->mode[k]) PTI_CUDA(cudaStreamWaitEvent(s, arr->mode[k], 0), mod);
     }
-    inv.reset();
+    PTI_TRY(ensure_err_word(t, s));
+    PlanGatherArgs g{};
+    g.n = n;
+    g.nb = nb;
+    g.nmodes = N;
+    g.mode = mode;
+    g.sb = t->sb;
+    g.bperm = bperm.as<uint32_t>();
+    g.order = order.as<uint32_t>();
+    g.tile_block = P.tile_block.as<uint32_t>();
+    g.lblk = P.lblk.as<uint16_t>();
+    g.vals_in = t->vals.as<float>();
+    for (uint32_t k = 0; k < N; ++k) {
+        PTI_CUDA(P.binds[k].alloc(padded(nb * 4), s), mod);
+        PTI_CUDA(P.einds[k].alloc(padded(n), s), mod);
+        g.dims[k] = t->ndims[k];
+        g.binds_in[k] = t->binds[k].as<uint32_t>();
+        g.einds_in[k] = t->einds[k].as<uint8_t>();
+        g.binds[k] = P.binds[k].as<uint32_t>();
+        g.einds[k] = P.einds[k].as<uint8_t>();
+    }
+    PTI_CUDA(P.vals.alloc(padded(n * 4), s), mod);
+    PTI_CUDA(P.recs.alloc(padded(n * 16), s), mod);
+    if (N == 4) {
+        PTI_CUDA(P.bquad.alloc(padded(nb * 16), s), mod);
+        PTI_CUDA(P.rvals.alloc(padded(n * 4), s), mod);
+    }
+    g.vals = P.vals.as<float>();
+    g.bquad = P.bquad.as<uint4>();
+    g.recs = P.recs.as<uint4>();
+    g.rvals = P.rvals.as<float>();
+    g.err = err_word(t);
+    plan_blocks_kernel<<<grid_n(nb), 256, 0, s>>>(g);
+    if (N == 2) plan_nonzeros_kernel<2><<<grid_n(n), 256, 0, s>>>(g);
+    else if (N == 3) plan_nonzeros_kernel<3><<<grid_n(n), 256, 0, s>>>(g);
+    else plan_nonzeros_kernel<4><<<grid_n(n), 256, 0, s>>>(g);
     PTI_CUDA(cudaGetLastError(), mod);
     P.ready = true;
     return 0;
