@@ -17,6 +17,8 @@
 // cptr follows the reference's greedy chunk rule (convert.c:737-742,805-815),
 // which only depends on the blocks of one kernel and the size of the last
 // block of the previous kernel, so one thread walks each kernel.
+#include <type_traits>
+
 #include "primitives.cuh"
 #include "tensor.cuh"
 
@@ -70,6 +72,84 @@ __device__ __forceinline__ U128 hicoo_key(const KeySpec &ks, uint64_t z)
     return k;
 }
 
+// Bits of x moved to every N-th position (x < 2^21 for N = 3, 2^16 for N = 4),
+// and back.
+template <int N>
+__device__ __forceinline__ uint64_t spread_bits(uint64_t x)
+{
+    if constexpr (N == 3) {
+        x = (x | x << 32) & 0x001F00000000FFFFull;
+        x = (x | x << 16) & 0x001F0000FF0000FFull;
+        x = (x | x << 8) & 0x100F00F00F00F00Full;
+        x = (x | x << 4) & 0x10C30C30C30C30C3ull;
+        x = (x | x << 2) & 0x1249249249249249ull;
+    } else {
+        x = (x | x << 24) & 0x000000FF000000FFull;
+        x = (x | x << 12) & 0x000F000F000F000Full;
+        x = (x | x << 6) & 0x0303030303030303ull;
+        x = (x | x << 3) & 0x1111111111111111ull;
+    }
+    return x;
+}
+template <int N>
+__device__ __forceinline__ uint32_t gather_bits(uint64_t x)
+{
+    if constexpr (N == 3) {
+        x &= 0x1249249249249249ull;
+        x = (x | x >> 2) & 0x10C30C30C30C30C3ull;
+        x = (x | x >> 4) & 0x100F00F00F00F00Full;
+        x = (x | x >> 8) & 0x001F0000FF0000FFull;
+        x = (x | x >> 16) & 0x001F00000000FFFFull;
+        x = (x | x >> 32) & 0x00000000001FFFFFull;
+    } else {
+        x &= 0x1111111111111111ull;
+        x = (x | x >> 3) & 0x0303030303030303ull;
+        x = (x | x >> 6) & 0x000F000F000F000Full;
+        x = (x | x >> 12) & 0x000000FF000000FFull;
+        x = (x | x >> 24) & 0x000000000000FFFFull;
+    }
+    return (uint32_t)x;
+}
+
+// Keys that hold every coordinate bit in one word: total <= 64 bits, and the
+// Morton part takes all low bits (mbits_per_mode == sk <= 21 or 16).  The
+// sorted keys then give back the coordinates, so that neither they nor the
+// blocks are gathered through the permutation.
+static bool whole_keys(const KeySpec &ks, uint32_t total)
+{
+    return total <= 64 && ks.mbits_per_mode == ks.sk && ks.sk <= (ks.nmodes == 3 ? 21u : 16u);
+}
+
+template <int N>
+__global__ void __launch_bounds__(256) make_whole_keys_kernel(KeySpec ks, uint64_t n, uint64_t *keys, uint32_t *vals)
+{
+    const uint32_t low = (1u << ks.sk) - 1u;
+    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256) {
+        uint64_t hi = 0, lo = 0;
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            const uint32_t c = ks.inds[m][i];
+            hi = hi << ks.kbits[m] | c >> ks.sk;
+            lo |= spread_bits<N>(c & low) << (N - 1 - m);
+        }
+        keys[i] = N * ks.sk < 64 ? hi << (N * ks.sk) | lo : lo;
+        vals[i] = (uint32_t)i;
+    }
+}
+
+// Coordinates of mode 0..N-1 from a whole key.
+template <int N>
+__device__ __forceinline__ void key_coords(const KeySpec &ks, uint64_t key, uint32_t (&c)[N])
+{
+    uint64_t hi = N * ks.sk < 64 ? key >> (N * ks.sk) : 0;
+    const uint64_t lo = N * ks.sk < 64 ? key & (((uint64_t)1 << (N * ks.sk)) - 1) : key;
+#pragma unroll
+    for (int m = N - 1; m >= 0; --m) {
+        c[m] = (uint32_t)(hi & (((uint64_t)1 << ks.kbits[m]) - 1)) << ks.sk | gather_bits<N>(lo >> (N - 1 - m));
+        hi >>= ks.kbits[m];
+    }
+}
+
 __global__ void make_keys_kernel(KeySpec ks, uint64_t n, int word, const uint32_t *perm, uint64_t *keys,
                                  uint32_t *vals)
 {
@@ -106,6 +186,75 @@ __global__ void gather_sorted_kernel(GatherArgs a, uint64_t n)
             }
         a.svals[z] = a.vals[p];
     }
+}
+
+// The same from whole keys; the sorted coordinates only where they are asked for.
+template <int N>
+__global__ void __launch_bounds__(256) unpack_sorted_kernel(KeySpec ks, const uint64_t *keys, GatherArgs a, uint64_t n)
+{
+    const uint32_t emask = (1u << a.sb) - 1u;
+    for (uint64_t z = (uint64_t)blockIdx.x * 256 + threadIdx.x; z < n; z += (uint64_t)gridDim.x * 256) {
+        a.svals[z] = a.vals[a.perm[z]];
+        uint32_t c[N];
+        key_coords<N>(ks, keys[z], c);
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            if (a.sinds[m]) a.sinds[m][z] = c[m];
+            a.einds[m][z] = (uint8_t)(c[m] & emask);
+        }
+    }
+}
+
+// Whole keys: blocks and kernels start where the bits above the element
+// offsets, or above the Morton part, change (both counts of bits are below 64).
+struct KeyChange {
+    const uint64_t *keys;
+    uint32_t shift;
+    __device__ uint32_t operator()(uint64_t z) const
+    {
+        return z == 0 || keys[z] >> shift != keys[z - 1] >> shift ? 1u : 0u;
+    }
+};
+
+template <int N>
+struct KeyBlockOut {
+    KeySpec ks;
+    uint32_t sb;
+    const uint64_t *keys;
+    uint64_t *bptr;
+    uint32_t *binds[N];
+    __device__ void operator()(uint64_t z, uint32_t prefix, uint32_t flag) const
+    {
+        if (!flag) return;
+        bptr[prefix] = z;
+        uint32_t c[N];
+        key_coords<N>(ks, keys[z], c);
+#pragma unroll
+        for (int m = 0; m < N; ++m) binds[m][prefix] = c[m] >> sb;
+    }
+};
+
+struct KeyKernelFlag {
+    const uint64_t *keys, *bptr;
+    uint32_t shift;
+    __device__ uint32_t operator()(uint64_t b) const
+    {
+        if (b == 0) return 1u;
+        const uint64_t z = bptr[b];
+        return shift < 64 && keys[z] >> shift != keys[z - 1] >> shift ? 1u : 0u;
+    }
+};
+
+template <int N>
+__global__ void key_kernel_coords_kernel(uint64_t nk, KeySpec ks, const uint64_t *keys, const uint64_t *kptr,
+                                         const uint64_t *bptr, uint32_t *kc)
+{
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nk) return;
+    uint32_t c[N];
+    key_coords<N>(ks, keys[bptr[kptr[k]]], c);
+#pragma unroll
+    for (int m = 0; m < N; ++m) kc[m * nk + k] = c[m] >> ks.sk;
 }
 
 // 1 if nonzero z of the sorted tensor starts a new block (z == 0 or block
@@ -255,11 +404,11 @@ struct ConvertExtras {
     DevBuf kptr;      // uint64 [nk+1]
     DevBuf cptr;      // uint64 [nc]
     DevBuf kcoords;   // uint32 [nmodes][nk]
-    std::array<DevBuf, kMaxModes> sinds;  // the COO indices in HiCOO order
-    DevBuf svals;
+    std::array<DevBuf, kMaxModes> sinds;  // the COO indices in HiCOO order, where asked for
 };
 
-int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8_t sk, uint8_t sc,
+// sorted_coo: the caller wants the COO arrays in HiCOO order (ex.sinds, ex.svals).
+int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8_t sk, uint8_t sc, bool sorted_coo,
                    ConvertExtras &ex, cudaStream_t s)
 {
     const char *mod = "B200 HiSpTns Convert";
@@ -293,7 +442,10 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
     PTI_CUDA(perm.alloc(padded(n * 4), s), mod);
     PTI_TRY(rs.alloc(n, s));
     const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 32);
-    make_keys_kernel<<<grid, 256, 0, s>>>(ks, n, 0, nullptr, keys.as<uint64_t>(), perm.as<uint32_t>());
+    const bool whole = whole_keys(ks, total);
+    if (!whole) make_keys_kernel<<<grid, 256, 0, s>>>(ks, n, 0, nullptr, keys.as<uint64_t>(), perm.as<uint32_t>());
+    else if (N == 3) make_whole_keys_kernel<3><<<grid, 256, 0, s>>>(ks, n, keys.as<uint64_t>(), perm.as<uint32_t>());
+    else make_whole_keys_kernel<4><<<grid, 256, 0, s>>>(ks, n, keys.as<uint64_t>(), perm.as<uint32_t>());
     PTI_CUDA(cudaGetLastError(), mod);
     PTI_TRY(radix_sort_pairs(keys, perm, n, total < 64 ? (int)total : 64, rs, s));
     if (total > 64) {
@@ -301,7 +453,7 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
         PTI_CUDA(cudaGetLastError(), mod);
         PTI_TRY(radix_sort_pairs(keys, perm, n, (int)(total - 64), rs, s));
     }
-    keys.reset();
+    if (!whole) keys.reset();
     rs = RadixScratch();
 
     // Sorted COO, einds and values.
@@ -319,18 +471,18 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
     ga.perm = perm.as<uint32_t>();
     ga.vals = coo->vals.as<float>();
     for (uint32_t m = 0; m < N; ++m) {
-        PTI_CUDA(ex.sinds[m].alloc(padded(n * 4), s), mod);
+        if (sorted_coo || !whole) PTI_CUDA(ex.sinds[m].alloc(padded(n * 4), s), mod);
         PTI_CUDA(h->einds[m].alloc(padded(n), s), mod);
         ga.inds[m] = coo->inds[m].as<uint32_t>();
         ga.sinds[m] = ex.sinds[m].as<uint32_t>();
         ga.einds[m] = h->einds[m].as<uint8_t>();
     }
-    PTI_CUDA(ex.svals.alloc(padded(n * 4), s), mod);
     PTI_CUDA(h->vals.alloc(padded(n * 4), s), mod);
     ga.svals = h->vals.as<float>();
-    gather_sorted_kernel<<<grid, 256, 0, s>>>(ga, n);
+    if (!whole) gather_sorted_kernel<<<grid, 256, 0, s>>>(ga, n);
+    else if (N == 3) unpack_sorted_kernel<3><<<grid, 256, 0, s>>>(ks, keys.as<uint64_t>(), ga, n);
+    else unpack_sorted_kernel<4><<<grid, 256, 0, s>>>(ks, keys.as<uint64_t>(), ga, n);
     PTI_CUDA(cudaGetLastError(), mod);
-    PTI_CUDA(cudaMemcpyAsync(ex.svals.ptr, h->vals.ptr, n * 4, cudaMemcpyDeviceToDevice, s), mod);
     perm.reset();
 
     // Blocks: bptr, binds.  Upper bound nb <= n until counted.
@@ -353,7 +505,15 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
     }
     bo.bptr = bptr_full.as<uint64_t>();
     uint32_t nb32 = 0;
-    PTI_TRY((exclusive_scan<uint32_t>(nbf, bo, n, scan_tmp.as<uint32_t>(), &nb32, s)));
+    auto key_blocks = [&](auto n_modes) -> int {
+        constexpr int M = decltype(n_modes)::value;
+        KeyBlockOut<M> kb{ks, sb, keys.as<uint64_t>(), bptr_full.as<uint64_t>(), {}};
+        for (int m = 0; m < M; ++m) kb.binds[m] = binds_full[m].as<uint32_t>();
+        return exclusive_scan<uint32_t>(KeyChange{keys.as<uint64_t>(), N * sb}, kb, n, scan_tmp.as<uint32_t>(), &nb32, s);
+    };
+    if (!whole) PTI_TRY((exclusive_scan<uint32_t>(nbf, bo, n, scan_tmp.as<uint32_t>(), &nb32, s)));
+    else if (N == 3) PTI_TRY(key_blocks(std::integral_constant<int, 3>{}));
+    else PTI_TRY(key_blocks(std::integral_constant<int, 4>{}));
     const uint64_t nb = nb32;
     h->nb = nb;
     PTI_CUDA(cudaMemcpyAsync(bptr_full.as<uint64_t>() + nb, &n, 8, cudaMemcpyHostToDevice, s), mod);
@@ -376,8 +536,12 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
     DevBuf kptr_full;
     PTI_CUDA(kptr_full.alloc(padded((nb + 1) * 8), s), mod);
     uint32_t nk32 = 0;
-    PTI_TRY((exclusive_scan<uint32_t>(nkf, KernelOut{kptr_full.as<uint64_t>()}, nb, scan_tmp.as<uint32_t>(),
-                                      &nk32, s)));
+    if (!whole)
+        PTI_TRY((exclusive_scan<uint32_t>(nkf, KernelOut{kptr_full.as<uint64_t>()}, nb, scan_tmp.as<uint32_t>(),
+                                          &nk32, s)));
+    else
+        PTI_TRY((exclusive_scan<uint32_t>(KeyKernelFlag{keys.as<uint64_t>(), h->bptr.as<uint64_t>(), N * sk},
+                                          KernelOut{kptr_full.as<uint64_t>()}, nb, scan_tmp.as<uint32_t>(), &nk32, s)));
     const uint64_t nk = nk32;
     ex.nk = nk;
     PTI_CUDA(ex.kptr.alloc(padded((nk + 1) * 8), s), mod);
@@ -411,8 +575,15 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
     KeySpec kcs = ks;
     for (uint32_t m = 0; m < N; ++m) kcs.inds[m] = ex.sinds[m].as<uint32_t>();
     PTI_CUDA(ex.kcoords.alloc(padded(nk * N * 4), s), mod);
-    kernel_coords_kernel<<<ceil_div(nk, 256), 256, 0, s>>>(nk, N, sk, ex.kptr.as<uint64_t>(), h->bptr.as<uint64_t>(),
-                                                            kcs, ex.kcoords.as<uint32_t>());
+    if (!whole)
+        kernel_coords_kernel<<<ceil_div(nk, 256), 256, 0, s>>>(nk, N, sk, ex.kptr.as<uint64_t>(),
+                                                                h->bptr.as<uint64_t>(), kcs, ex.kcoords.as<uint32_t>());
+    else if (N == 3)
+        key_kernel_coords_kernel<3><<<ceil_div(nk, 256), 256, 0, s>>>(
+            nk, ks, keys.as<uint64_t>(), ex.kptr.as<uint64_t>(), h->bptr.as<uint64_t>(), ex.kcoords.as<uint32_t>());
+    else
+        key_kernel_coords_kernel<4><<<ceil_div(nk, 256), 256, 0, s>>>(
+            nk, ks, keys.as<uint64_t>(), ex.kptr.as<uint64_t>(), h->bptr.as<uint64_t>(), ex.kcoords.as<uint32_t>());
     PTI_CUDA(cudaGetLastError(), mod);
     unsigned long long mxh = 0;
     PTI_CUDA(cudaMemcpyAsync(&mxh, mx.ptr, 8, cudaMemcpyDeviceToHost, s), mod);
@@ -455,7 +626,7 @@ int ptiSparseTensorToHiCOO(ptiSparseTensorHiCOO *hitsr, ptiNnzIndex *max_nnzb, p
     ptiB200Tensor coo, h;
     PTI_TRY(upload_coo(&coo, tsr, s));
     ConvertExtras ex;
-    PTI_TRY(convert_device(&coo, &h, sb_bits, sk_bits, sc_bits, ex, s));
+    PTI_TRY(convert_device(&coo, &h, sb_bits, sk_bits, sc_bits, true, ex, s));
     const uint32_t N = tsr->nmodes;
     const uint64_t n = tsr->nnz, nb = h.nb, nk = ex.nk;
 
@@ -463,7 +634,7 @@ int ptiSparseTensorToHiCOO(ptiSparseTensorHiCOO *hitsr, ptiNnzIndex *max_nnzb, p
     // The caller's COO is left sorted in HiCOO order, as in the reference.
     for (uint32_t m = 0; m < N; ++m)
         PTI_CUDA(cudaMemcpyAsync(tsr->inds[m].data, ex.sinds[m].ptr, n * 4, cudaMemcpyDeviceToHost, s), mod);
-    PTI_CUDA(cudaMemcpyAsync(tsr->values.data, ex.svals.ptr, n * 4, cudaMemcpyDeviceToHost, s), mod);
+    PTI_CUDA(cudaMemcpyAsync(tsr->values.data, h.vals.ptr, n * 4, cudaMemcpyDeviceToHost, s), mod);
     for (uint32_t m = 0; m < N; ++m) tsr->sortorder[m] = m;
 
     PTI_TRY(alloc_nnz_vector(&hitsr->bptr, nb + 1));
@@ -557,7 +728,7 @@ int ptiB200ConvertToHiCOO(ptiB200Tensor **out, ptiB200Tensor *coo, ptiElementInd
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto *h = new ptiB200Tensor();
     ConvertExtras ex;
-    int r = convert_device(coo, h, sb_bits, sk_bits, sc_bits, ex, s);
+    int r = convert_device(coo, h, sb_bits, sk_bits, sc_bits, false, ex, s);
     if (r == 0) r = finish_hicoo_layout(h, s);
     if (r) {
         delete h;
