@@ -222,19 +222,25 @@ uint32_t *err_word(ptiB200Tensor *t);
 int mttkrp_scheduled(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t R, uint32_t stride,
                      const uint32_t *mats_order, uint32_t mode, float *out, cudaStream_t s,
                      const float *vals_override);
-bool schedule_supported(const ptiB200Tensor *t, uint32_t R, uint32_t stride);
+bool schedule_supported(const ptiB200Tensor *t, uint32_t mode, uint32_t R, uint32_t stride, bool own_vals,
+                        cudaStream_t s);
 
-// The output-privatised kernels (sched.cu) cover orders 2-4, R <= 128 and
-// (HiCOO) factors of fewer than 2^32 elements; HIPARTI_B200_SCHEDULE=0 selects
-// the direct-atomic kernels instead.
-static bool use_schedule(const ptiB200Tensor *t, uint32_t R, uint32_t stride)
+// The output-privatised kernels (sched.cu) cover every order of a COO tensor,
+// orders 2-4 of a HiCOO tensor with factors of fewer than 2^32 elements, and
+// any rank.  HIPARTI_B200_SCHEDULE=0 selects the direct-atomic kernels, where
+// every product is an atomic of its own: they are left for HiCOO tensors of 5
+// or more modes and the cases schedule_supported() names.  (3M Zipf nonzeros of
+// a 4-D COO tensor, R = 150, every mode: direct 9.4 ms, scheduled 1.27; 2M Zipf
+// in HiCOO, R = 130, BF16: 3.29 and 0.42; 3M uniform 5-D, R = 32: 0.77 and 0.47.)
+static bool use_schedule(const ptiB200Tensor *t, uint32_t mode, uint32_t R, uint32_t stride, bool own_vals,
+                         cudaStream_t s)
 {
     static int env = -1;
     if (env < 0) {
         const char *e = std::getenv("HIPARTI_B200_SCHEDULE");
         env = (e && e[0] == '0') ? 0 : 1;
     }
-    return env == 1 && schedule_supported(t, R, stride);
+    return env == 1 && schedule_supported(t, mode, R, stride, own_vals, s);
 }
 
 int mttkrp_device(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t R, uint32_t stride,
@@ -267,7 +273,7 @@ int mttkrp_device(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t R,
     PTI_CUDA(cudaMemsetAsync(out, 0, (size_t)t->ndims[mode] * stride * sizeof(float), s), mod);
     if (t->nnz == 0) return 0;
     const int G = group_lanes(R);
-    if (use_schedule(t, R, stride)) {
+    if (use_schedule(t, mode, R, stride, vals_override == nullptr, s)) {
         PTI_TRY(prepare_mode(t, mode, s, arr));
         if (arr && arr->all) PTI_CUDA(cudaStreamWaitEvent(s, arr->all, 0), mod);
         return mttkrp_scheduled(t, mats, ft, R, stride, mats_order, mode, out, s, vals_override);
@@ -864,6 +870,8 @@ int ptiB200MTTKRP(ptiB200Tensor *t, const void *const *dev_mats, int factor_type
 int ptiB200Prepare(ptiB200Tensor *t, ptiIndex mode, void *stream)
 {
     PTI_CHECK(t, PTIERR_VALUE_ERROR, "B200 Prepare", "null handle");
+    PTI_CHECK(t->nmodes <= 4 || t->nnz == 0, PTIERR_VALUE_ERROR, "B200 Prepare",
+              "schedules are prepared ahead for orders up to 4");
     return pti::prepare_mode(t, mode, static_cast<cudaStream_t>(stream));
 }
 

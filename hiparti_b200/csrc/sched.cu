@@ -21,6 +21,7 @@
 // into global memory once per run of equal rows (16-byte vector atomics); a
 // row shared by neighbouring groups is merged in shared memory first, so a hot
 // row costs one global add per tile instead of one per nonzero.
+#include <mutex>
 #include <type_traits>
 
 #include "kutil.cuh"
@@ -37,7 +38,7 @@ namespace pti {
 // four modes of a uniform 4-D tensor of 5M nonzeros at R = 32.  BF16 rows keep
 // 2048, as their walk feeds on the L1 that the fourth CTA's shared memory
 // would take (574 us, and 609 with 1024, for 5M Zipf nonzeros at R = 64).
-constexpr uint32_t coo_tile(int words, int cpl) { return cpl == 8 || words <= 4 ? 2048u : 8192u / words; }
+constexpr uint32_t coo_tile(int words, int cpl) { return cpl == 8 || words <= 4 ? 2048u : 8192u / words & ~3u; }
 constexpr int kHiTile = kPlanTile; // nonzeros per CTA (HiCOO kernel)
 constexpr int kSchedThreads = 256;
 
@@ -70,9 +71,10 @@ __device__ __forceinline__ uint32_t round16(uint32_t x) { return (x + 15u) & ~15
 
 // Words per packed nonzero record {output row, operand rows..., value},
 // rounded up to 16 bytes.
+constexpr int rec_words(int nin) { return (nin + 2 + 3) / 4 * 4; }
 template <int NIN>
 struct Rec {
-    static constexpr int words = ((NIN + 2 + 3) / 4) * 4;
+    static constexpr int words = rec_words(NIN);
 };
 
 // Columns of one operand row held by a lane: CPL consecutive columns, loaded
@@ -990,10 +992,9 @@ static unsigned grid_n(uint64_t n)
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 32));
 }
 
-int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals *arr)
+static int build_plan(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals *arr)
 {
     const char *mod = "B200 Prepare";
-    PTI_CHECK(mode < t->nmodes, PTIERR_VALUE_ERROR, mod, "mode out of range");
     const uint32_t N = t->nmodes;
     const uint64_t n = t->nnz;
     PTI_CHECK(n < 0xFFFFFFFFull, PTIERR_VALUE_ERROR, mod, "too many nonzeros");
@@ -1001,7 +1002,6 @@ int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals
     if (!t->hicoo) {
         CooModePlan &P = t->coo_plan[mode];
         if (P.ready) return 0;
-        PTI_CHECK(N <= 4, PTIERR_VALUE_ERROR, mod, "COO schedules cover orders up to 4");
         DevBuf keys, perm;
         RadixScratchT<uint32_t> rs;
         PTI_CUDA(keys.alloc(padded(n * 4), s), mod);
@@ -1010,7 +1010,7 @@ int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals
         iota_keys_kernel<<<grid_n(n), 256, 0, s>>>(t->inds[mode].as<uint32_t>(), n, keys.as<uint32_t>(),
                                                    perm.as<uint32_t>());
         PTI_TRY(radix_sort_pairs(keys, perm, n, (int)bits_for_count(t->ndims[mode]), rs, s));
-        const int RW = N <= 3 ? 4 : 8;
+        const int RW = rec_words((int)N - 1);
         PTI_CUDA(P.recs.alloc(padded(n * RW * 4), s), mod);
         PackArgs pa{};
         pa.nin = N - 1;
@@ -1121,6 +1121,43 @@ int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals
     return 0;
 }
 
+bool plan_ready(const ptiB200Tensor *t, uint32_t mode)
+{
+    return t->hicoo ? t->hicoo_plan[mode].ready : t->coo_plan[mode].ready;
+}
+
+static bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
+// Builds the schedule of `mode` on first use.  The first call on a handle may
+// come from any thread and stream, so the build is under the handle's lock and
+// leaves an event behind: a call on another stream than the building one waits
+// for it on the device.  (A capturing stream cannot wait for work outside its
+// capture; a program captures after the schedules are built.)
+int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals *arr)
+{
+    const char *mod = "B200 Prepare";
+    PTI_CHECK(mode < t->nmodes, PTIERR_VALUE_ERROR, mod, "mode out of range");
+    if (t->nnz == 0) return build_plan(t, mode, s, arr);
+    std::lock_guard<std::mutex> lock(t->plan_mu);
+    PlanOrder &o = t->plan_order[mode];
+    if (plan_ready(t, mode)) {
+        if (o.event && s != o.stream && !capturing(s)) PTI_CUDA(cudaStreamWaitEvent(s, o.event, 0), mod);
+        return 0;
+    }
+    PTI_TRY(ensure_err_word(t, s));
+    PTI_TRY(build_plan(t, mode, s, arr));
+    if (!capturing(s)) {
+        if (!o.event) PTI_CUDA(cudaEventCreateWithFlags(&o.event, cudaEventDisableTiming), mod);
+        PTI_CUDA(cudaEventRecord(o.event, s), mod);
+        o.stream = s;
+    }
+    return 0;
+}
+
 // ---------------------------------------------------------------------------
 // Launch
 // ---------------------------------------------------------------------------
@@ -1142,7 +1179,8 @@ static int launch_coo(const SchedArgs &a, const uint32_t *recs, cudaStream_t s)
 {
     constexpr uint32_t RW = Rec<NIN>::words, kTile = coo_tile(RW, CPL);
     constexpr size_t smem_max = (size_t)kTile * RW * 4 + (size_t)kSchedThreads * CPL * 4;
-    constexpr int UU = NIN == 3 && U > 2 ? 2 : U;  // 4-D records hold more registers per nonzero
+    // more operands hold more registers per nonzero in flight
+    constexpr int UU = NIN > 4 ? 1 : (NIN >= 3 && U > 2 ? 2 : U);
     auto k = coo_sched_kernel<G, CPL, UU, PTI_COO_MINB, FT, NIN>;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max) != cudaSuccess)
         return PTIERR_CUDA_ERROR;
@@ -1247,6 +1285,17 @@ static int launch_r(bool hicoo, bool wide, const SchedArgs &a, const uint32_t *r
     return launch_coo<32, 4, 2, FT, NIN>(a, recs, s);
 }
 
+// COO schedules of 5 to 8 modes: 4 columns per lane.
+template <class FT, int NIN>
+static int launch_high(const SchedArgs &a, const uint32_t *recs, cudaStream_t s)
+{
+    if (a.R <= 8) return launch_coo<2, 4, 2, FT, NIN>(a, recs, s);
+    if (a.R <= 16) return launch_coo<4, 4, 2, FT, NIN>(a, recs, s);
+    if (a.R <= 32) return launch_coo<8, 4, 2, FT, NIN>(a, recs, s);
+    if (a.R <= 64) return launch_coo<16, 4, 2, FT, NIN>(a, recs, s);
+    return launch_coo<32, 4, 2, FT, NIN>(a, recs, s);
+}
+
 template <class FT>
 static int launch_n(int nin, bool hicoo, bool wide, const SchedArgs &a, const uint32_t *recs, unsigned ntiles,
                     cudaStream_t s)
@@ -1254,13 +1303,35 @@ static int launch_n(int nin, bool hicoo, bool wide, const SchedArgs &a, const ui
     switch (nin) {
         case 1: return launch_r<FT, 1>(hicoo, wide, a, recs, ntiles, s);
         case 2: return launch_r<FT, 2>(hicoo, wide, a, recs, ntiles, s);
-        default: return launch_r<FT, 3>(hicoo, wide, a, recs, ntiles, s);
+        case 3: return launch_r<FT, 3>(hicoo, wide, a, recs, ntiles, s);
+        case 4: return launch_high<FT, 4>(a, recs, s);
+        case 5: return launch_high<FT, 5>(a, recs, s);
+        case 6: return launch_high<FT, 6>(a, recs, s);
+        default: return launch_high<FT, 7>(a, recs, s);
     }
 }
 
-bool schedule_supported(const ptiB200Tensor *t, uint32_t R, uint32_t stride)
+// Ranks above kPanel run as panels of kPanel columns (the last one narrower),
+// one launch each over the same schedule, because a lane group covers at most
+// 32 lanes x 4 columns and holds one partial row.  COO records take any order;
+// the HiCOO kernels hold three operand rows per record.
+constexpr uint32_t kPanel = 128;
+
+bool schedule_supported(const ptiB200Tensor *t, uint32_t mode, uint32_t R, uint32_t stride, bool own_vals,
+                        cudaStream_t s)
 {
-    if (!(t->nmodes >= 2 && t->nmodes <= 4 && R >= 1 && R <= 128)) return false;
+    if (t->nmodes < 2 || t->nmodes > (t->hicoo ? 4u : (uint32_t)kMaxModes) || R < 1) return false;
+    if (t->nnz >= 0xFFFFFFFFull && (t->nmodes > 4 || R > kPanel)) return false;  // schedules index nonzeros by 32 bits
+    // One launch of the direct kernel against one per panel: COO, R = 150, three
+    // modes, 5,000 nonzeros 51 us against 65, 20,000 Zipf 64 against 65, 50,000
+    // Zipf 126 against 64.  (The direct HiCOO kernel is slower at every size.)
+    constexpr uint64_t kDirectBelow = 16384;
+    if (!t->hicoo && R > kPanel && t->nnz < kDirectBelow) return false;
+    // Above 4 modes or one panel the direct kernels stay the choice where a
+    // schedule would add state that such calls did not have: substituted
+    // values (one reordered copy per mode and handle), and a first use inside
+    // a stream capture (the schedule's memory would belong to the graph).
+    if ((t->nmodes > 4 || R > kPanel) && (!own_vals || (!plan_ready(t, mode) && capturing(s)))) return false;
     // the HiCOO kernel addresses factor rows by 32-bit element offsets
     if (t->hicoo)
         for (uint32_t m = 0; m < t->nmodes; ++m)
@@ -1333,9 +1404,17 @@ int mttkrp_scheduled(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t
     bool wide = ft == PTI_B200_BF16 && stride % 8 == 0;
     for (uint32_t k = 0; k < N && wide; ++k)
         if (k != mode && ((uintptr_t)mats[k] & 15) != 0) wide = false;
-    int r = ft == PTI_B200_F32 ? launch_n<float>((int)N - 1, t->hicoo, false, a, recs, ntiles, s)
-                               : launch_n<__nv_bfloat16>((int)N - 1, t->hicoo, wide, a, recs, ntiles, s);
-    PTI_CHECK(r == 0, r, mod, "kernel attribute setup failed");
+    const size_t esz = ft == PTI_B200_F32 ? 4 : 2;
+    for (uint32_t c0 = 0; c0 < R; c0 += kPanel) {
+        SchedArgs p = a;
+        p.R = std::min(R - c0, kPanel);
+        p.out = out + c0;
+        for (uint32_t i = 0; i + 1 < N; ++i)
+            p.in_mat[i] = static_cast<const unsigned char *>(a.in_mat[i]) + (size_t)c0 * esz;
+        const int r = ft == PTI_B200_F32 ? launch_n<float>((int)N - 1, t->hicoo, false, p, recs, ntiles, s)
+                                         : launch_n<__nv_bfloat16>((int)N - 1, t->hicoo, wide, p, recs, ntiles, s);
+        PTI_CHECK(r == 0, r, mod, "kernel attribute setup failed");
+    }
     PTI_CUDA(cudaGetLastError(), mod);
     return 0;
 }

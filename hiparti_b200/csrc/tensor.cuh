@@ -4,6 +4,7 @@
 
 #include <array>
 #include <memory>
+#include <mutex>
 
 namespace pti {
 
@@ -45,12 +46,26 @@ struct HicooModePlan {
 };
 
 // Per-mode schedule of a COO tensor: nonzeros sorted by the output-mode index,
-// packed as 16- or 32-byte records {out index, operand indices, value}.
+// packed as records of 16, 32 or 48 bytes {out index, operand indices, value}.
 struct CooModePlan {
     bool ready = false;
     DevBuf recs;                          // uint32 [nnz][4 or 8]
     DevBuf perm;                          // uint32 [nnz]: record j holds input nonzero perm[j]
     DevBuf alt_vals;                      // float [nnz]: caller-supplied values in record order
+};
+
+// Where a mode's schedule was built: the stream and an event recorded behind
+// the build, for first uses from several streams.
+struct PlanOrder {
+    cudaEvent_t event = nullptr;
+    cudaStream_t stream = nullptr;
+    PlanOrder() = default;
+    PlanOrder(const PlanOrder &) = delete;
+    PlanOrder &operator=(const PlanOrder &) = delete;
+    ~PlanOrder()
+    {
+        if (event) cudaEventDestroy(event);
+    }
 };
 
 // Fibers of a COO tensor along one mode (TTM / TTV): the nonzeros sorted by
@@ -97,6 +112,8 @@ struct ptiB200Tensor {
     std::array<pti::CooModePlan, pti::kMaxModes> coo_plan;
     std::array<pti::HicooModePlan, pti::kMaxModes> hicoo_plan;
     std::array<pti::FiberPlan, pti::kMaxModes> fiber_plan;
+    std::array<pti::PlanOrder, pti::kMaxModes> plan_order;
+    std::mutex plan_mu;  // held while a schedule is looked up or built
 };
 
 namespace pti {
