@@ -54,7 +54,9 @@ cudaStream_t sync_stream();
 // sync_stream().
 cudaStream_t copy_stream();
 // Two non-blocking side streams per device (0 is copy_stream()), for kernels
-// that run beside the caller's stream; created on first use.
+// that run beside the caller's stream; created on first use.  They have the
+// highest priority: what runs there is the longer chain, and its CTAs go ahead
+// of the waiting ones of a kernel that fills the GPU from the caller's stream.
 cudaStream_t side_stream(int which);
 
 // Stream-ordered device allocation from the runtime's default memory pool

@@ -53,7 +53,11 @@ cudaStream_t side_stream(int which)
     std::lock_guard<std::mutex> lock(mu);
     if ((int)streams.size() <= 2 * dev + 1) streams.resize(2 * dev + 2, nullptr);
     cudaStream_t &st = streams[2 * dev + (which & 1)];
-    if (!st) cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (!st) {
+        int low = 0, high = 0;
+        cudaDeviceGetStreamPriorityRange(&low, &high);
+        cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, high);
+    }
     return st;
 }
 

@@ -78,10 +78,11 @@ struct FiberPlan {
     DevBuf sind;                           // uint32 [nnz]: the mode's index, fiber order
     DevBuf sval;                           // float  [nnz]: values, fiber order
     DevBuf perm;                           // uint32 [nnz]: fiber-order position -> input nonzero
-    uint64_t nlong = 0;                    // fibers longer than one thread takes, up to the CTA limit
+    uint64_t nlong = 0;                    // fibers longer than a lane group takes, up to the CTA limit
     uint64_t nvlong = 0;                   // fibers longer than that, one CTA each
-    uint64_t nshort = 0;                   // fibers one thread takes
+    uint64_t nshort = 0;                   // fibers one lane group takes
     DevBuf short_fibs;                     // uint4 [nshort]: {fiber, length, first nonzero} by length class
+    DevBuf long_fibs;                      // uint4 [nlong]: the same for the nlong fibers
     DevBuf long_fibers;                    // uint32 [nfib]: the nlong fibers from the front, the nvlong from the back
 };
 

@@ -97,7 +97,7 @@ struct FiberOut {
 
 __global__ void set_last_t(uint64_t *fptr, uint64_t nfib, uint64_t nnz) { fptr[nfib] = nnz; }
 
-constexpr uint32_t kShortFiber = 64;      // longest fiber a single thread takes
+constexpr uint32_t kShortFiber = 64;      // longest fiber of ttm_short_kernel
 constexpr uint64_t kVLongFiber = 8192;    // longer fibers get a CTA each (ttm_vlong_kernel)
 
 // Fibers longer than kShortFiber: up to kVLongFiber nonzeros from the front of
@@ -112,7 +112,7 @@ __global__ void long_fibers_k(const uint64_t *fptr, uint64_t nfib, uint32_t *lis
     }
 }
 
-// Length class of every fiber for the one-thread-per-fiber kernel: 0 for one
+// Length class of every fiber for ttm_short_kernel: 0 for one
 // nonzero, c for 2^(c-1) < length <= 2^c up to kShortFiber, 7 above.
 __global__ void fiber_class_k(const uint64_t *fptr, uint64_t nfib, uint64_t *key, uint32_t *idx)
 {
@@ -124,8 +124,8 @@ __global__ void fiber_class_k(const uint64_t *fptr, uint64_t nfib, uint64_t *key
     }
 }
 
-// {fiber, length, first nonzero} of the fibers in `order`, for the kernel below.
-__global__ void pack_short_k(const uint64_t *fptr, const uint32_t *order, uint64_t n, uint4 *fibs)
+// {fiber, length, first nonzero} of the fibers in `order`, for the kernels below.
+__global__ void pack_fibers_k(const uint64_t *fptr, const uint32_t *order, uint64_t n, uint4 *fibs)
 {
     GRID_LOOP(i, n)
     {
@@ -135,56 +135,85 @@ __global__ void pack_short_k(const uint64_t *fptr, const uint32_t *order, uint64
     }
 }
 
-// One thread per short fiber, NC4 float4 column chunks (R <= 4 * NC4 <= 32).
-// The fibers come packed in order of their length class (so that a warp's
-// lanes walk fibers of similar lengths and finish together), each with its
-// first nonzero, so a thread starts from one coalesced 16-byte load.
-// U rows and Y rows are 16-byte aligned (ldu, ldy multiples of 4).
-template <int NC4>
+// Short fibers: a group of G lanes per fiber, lane l summing the 4 columns
+// from 4l (R <= 4 G <= 32), and kShortF fibers at a time in every group, whose
+// load chains (descriptor, index and value, row) overlap.  The fibers come
+// packed in order of their length class, so that a warp's groups finish
+// together.  U rows and Y rows are 16-byte aligned (ldu, ldy multiples of 4).
+//
+// A group reads and writes each row with one instruction: G lanes of 16 bytes
+// lie on one line, where a thread per fiber touched 32 lines with each of its
+// R / 4 loads and so spent four times as many L1 wavefronts at R = 16.
+// 5M Zipf nonzeros, R = 16, beside the kernels of the long fibers: 183 -> 135
+// us a mode.
+constexpr int kShortF = 4;
+
+template <int G>
 __global__ void __launch_bounds__(256) ttm_short_kernel(const uint4 *__restrict__ fibs, uint64_t nshort,
                                                         const uint32_t *__restrict__ sind,
                                                         const float *__restrict__ sval,
                                                         const float *__restrict__ U, uint32_t ldu,
                                                         float *__restrict__ Y, uint32_t ldy, uint32_t R)
 {
-    GRID_LOOP(i, nshort)
-    {
-        const uint4 fb = fibs[i];  // {fiber, length, first nonzero (64-bit)}
-        const uint64_t f = fb.x;
-        const uint64_t b = (uint64_t)fb.z | (uint64_t)fb.w << 32, e = b + fb.y;
-        float4 acc[NC4];
+    constexpr uint32_t kGroups = 256 / G;
+    const uint32_t lane = threadIdx.x % G, col = 4 * lane;
+    const uint64_t i0 = (uint64_t)blockIdx.x * (kGroups * kShortF) + threadIdx.x / G;
+    const bool mine = col < R;
+    uint4 fb[kShortF];  // {fiber, length, first nonzero (64-bit)}; length 0: none
+    uint32_t longest = 0;
 #pragma unroll
-        for (int c = 0; c < NC4; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t r = sind[b];
-        float x = sval[b];
-        for (uint64_t j = b; j < e; ++j) {
-            // the next nonzero's index and value load while this one is added
-            const uint32_t rn = j + 1 < e ? sind[j + 1] : 0u;
-            const float xn = j + 1 < e ? sval[j + 1] : 0.f;
-            const float4 *u = reinterpret_cast<const float4 *>(U + (size_t)r * ldu);
+    for (int k = 0; k < kShortF; ++k) {
+        const uint64_t i = i0 + (uint64_t)k * kGroups;
+        fb[k] = i < nshort ? fibs[i] : make_uint4(0u, 0u, 0u, 0u);
+        longest = max(longest, fb[k].y);
+    }
+    float4 acc[kShortF];
+    uint64_t b[kShortF];
+    uint32_t r[kShortF];
+    float x[kShortF];
 #pragma unroll
-            for (int c = 0; c < NC4; ++c) {
-                const float4 v = __ldg(u + c);
-                acc[c].x = __fadd_rn(acc[c].x, __fmul_rn(x, v.x));
-                acc[c].y = __fadd_rn(acc[c].y, __fmul_rn(x, v.y));
-                acc[c].z = __fadd_rn(acc[c].z, __fmul_rn(x, v.z));
-                acc[c].w = __fadd_rn(acc[c].w, __fmul_rn(x, v.w));
+    for (int k = 0; k < kShortF; ++k) {
+        acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        b[k] = (uint64_t)fb[k].z | (uint64_t)fb[k].w << 32;
+        r[k] = fb[k].y ? sind[b[k]] : 0u;
+        x[k] = fb[k].y ? sval[b[k]] : 0.f;
+    }
+    for (uint32_t j = 0; j < longest; ++j) {
+        float4 v[kShortF];
+        float xc[kShortF];
+#pragma unroll
+        for (int k = 0; k < kShortF; ++k) {
+            xc[k] = x[k];
+            if (j < fb[k].y && mine) v[k] = __ldg(reinterpret_cast<const float4 *>(U + (size_t)r[k] * ldu + col));
+        }
+        // the next nonzeros' indices and values load while these are added
+#pragma unroll
+        for (int k = 0; k < kShortF; ++k)
+            if (j + 1 < fb[k].y) {
+                r[k] = sind[b[k] + j + 1];
+                x[k] = sval[b[k] + j + 1];
             }
-            r = rn;
-            x = xn;
-        }
-        float4 *y = reinterpret_cast<float4 *>(Y + (size_t)f * ldy);
 #pragma unroll
-        for (int c = 0; c < NC4; ++c) {
-            float4 v = acc[c];
-            // columns at or beyond R (the U pad is not read as data): zero
-            if (4 * c + 0 >= (int)R) v.x = 0.f;
-            if (4 * c + 1 >= (int)R) v.y = 0.f;
-            if (4 * c + 2 >= (int)R) v.z = 0.f;
-            if (4 * c + 3 >= (int)R) v.w = 0.f;
-            y[c] = v;
-        }
-        for (uint32_t k = 4 * NC4; k < ldy; k += 4) y[k / 4] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < kShortF; ++k)
+            if (j < fb[k].y && mine) {
+                acc[k].x = __fadd_rn(acc[k].x, __fmul_rn(xc[k], v[k].x));
+                acc[k].y = __fadd_rn(acc[k].y, __fmul_rn(xc[k], v[k].y));
+                acc[k].z = __fadd_rn(acc[k].z, __fmul_rn(xc[k], v[k].z));
+                acc[k].w = __fadd_rn(acc[k].w, __fmul_rn(xc[k], v[k].w));
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < kShortF; ++k) {
+        if (!fb[k].y) continue;
+        float4 v = acc[k];
+        // columns at or beyond R (the U pad is not read as data): zero
+        if (col + 0 >= R) v.x = 0.f;
+        if (col + 1 >= R) v.y = 0.f;
+        if (col + 2 >= R) v.z = 0.f;
+        if (col + 3 >= R) v.w = 0.f;
+        float *y = Y + (size_t)fb[k].x * ldy;
+        if (col < ldy) *reinterpret_cast<float4 *>(y + col) = v;
+        for (uint32_t c = 4 * G + col; c < ldy; c += 4 * G) *reinterpret_cast<float4 *>(y + c) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
@@ -213,32 +242,41 @@ inline size_t long_smem_bytes(uint32_t W)
     return (size_t)kLongRowSlots * 32 * W * 4 + (size_t)kLongIdxSlots * 32 * 8;
 }
 
-// Position in a warp's stream of groups: fiber list[i], group k of its ng.
+// Position in a warp's stream of groups: fiber fibs[i] ({fiber, length, first
+// nonzero}), group k of its ng.  The following fiber's descriptor is loaded a
+// fiber ahead, so that stepping to it waits for nothing (three dependent loads
+// a fiber and stage otherwise: 191 -> 148 us a mode for 5M Zipf nonzeros).
 struct GroupCursor {
     uint64_t i, f, b, e, k, ng;
     bool live;
-    __device__ __forceinline__ void fiber(const uint64_t *fptr, const uint32_t *list, uint64_t nlong)
+    uint4 ahead;
+    __device__ __forceinline__ void start(const uint4 *fibs, uint64_t nlong)
+    {
+        ahead = i < nlong ? fibs[i] : make_uint4(0u, 0u, 0u, 0u);
+        take(fibs, nlong);
+    }
+    __device__ __forceinline__ void take(const uint4 *fibs, uint64_t nlong)
     {
         live = i < nlong;
         if (!live) return;
-        f = list[i];
-        b = fptr[f];
-        e = fptr[f + 1];
-        ng = (e - b + 31) / 32;
+        f = ahead.x;
+        b = (uint64_t)ahead.z | (uint64_t)ahead.w << 32;
+        e = b + ahead.y;
+        ng = (ahead.y + 31) / 32;
         k = 0;
+        if (i + gridDim.x < nlong) ahead = fibs[i + gridDim.x];
     }
-    __device__ __forceinline__ void next(const uint64_t *fptr, const uint32_t *list, uint64_t nlong)
+    __device__ __forceinline__ void next(const uint4 *fibs, uint64_t nlong)
     {
         if (++k == ng) {
             i += gridDim.x;
-            fiber(fptr, list, nlong);
+            take(fibs, nlong);
         }
     }
     __device__ __forceinline__ uint64_t first() const { return b + 32 * k; }  // first nonzero of the group
 };
 
-__global__ void __launch_bounds__(32) ttm_long_kernel(const uint64_t *__restrict__ fptr,
-                                                      const uint32_t *__restrict__ list, uint64_t nlong,
+__global__ void __launch_bounds__(32) ttm_long_kernel(const uint4 *__restrict__ fibs, uint64_t nlong,
                                                       const uint32_t *__restrict__ sind,
                                                       const float *__restrict__ sval, const float *__restrict__ U,
                                                       uint32_t ldu, uint32_t R, uint32_t W, float *__restrict__ Y,
@@ -256,9 +294,9 @@ __global__ void __launch_bounds__(32) ttm_long_kernel(const uint64_t *__restrict
     };
     // cursors of the three stages: sums (group g - D), rows (g), indices (g + D)
     GroupCursor cs{blockIdx.x}, cr{blockIdx.x}, ci{blockIdx.x};
-    cs.fiber(fptr, list, nlong);
-    cr.fiber(fptr, list, nlong);
-    ci.fiber(fptr, list, nlong);
+    cs.start(fibs, nlong);
+    cr.start(fibs, nlong);
+    ci.start(fibs, nlong);
     float acc = 0.f;
     // ring slots of stream group g: row slot g mod (D+1), index slot g mod (2D+2)
     uint32_t r13 = kLongRowSlots - kLongD % kLongRowSlots, r26 = kLongIdxSlots - kLongD;  // g = -D
@@ -273,8 +311,25 @@ __global__ void __launch_bounds__(32) ttm_long_kernel(const uint64_t *__restrict
             const float *rows = su + (size_t)wrap(r13 + 1, kLongRowSlots) * 32 * W;
             const float *xs = sx + wrap(r26 + (kLongIdxSlots - kLongD), kLongIdxSlots) * 32;
             if ((uint32_t)lane < R) {
+                if (cnt == 32) {  // straight-line: only the additions wait for one another
+#pragma unroll
+                    for (int t0 = 0; t0 < 32; t0 += 16) {
+                        float p[16];
+#pragma unroll
+                        for (int t = 0; t < 16; t += 4) {
+                            const float4 x4 = *reinterpret_cast<const float4 *>(xs + t0 + t);
+                            p[t] = __fmul_rn(x4.x, rows[(size_t)(t0 + t) * W + lane]);
+                            p[t + 1] = __fmul_rn(x4.y, rows[(size_t)(t0 + t + 1) * W + lane]);
+                            p[t + 2] = __fmul_rn(x4.z, rows[(size_t)(t0 + t + 2) * W + lane]);
+                            p[t + 3] = __fmul_rn(x4.w, rows[(size_t)(t0 + t + 3) * W + lane]);
+                        }
+#pragma unroll
+                        for (int t = 0; t < 16; ++t) acc = __fadd_rn(acc, p[t]);
+                    }
+                } else {
 #pragma unroll 8
-                for (int t = 0; t < cnt; ++t) acc = __fadd_rn(acc, __fmul_rn(xs[t], rows[(size_t)t * W + lane]));
+                    for (int t = 0; t < cnt; ++t) acc = __fadd_rn(acc, __fmul_rn(xs[t], rows[(size_t)t * W + lane]));
+                }
             }
             if (cs.k + 1 == cs.ng) {  // the fiber's last group: its row of Y
                 float *y = Y + (size_t)cs.f * ldy;
@@ -282,7 +337,7 @@ __global__ void __launch_bounds__(32) ttm_long_kernel(const uint64_t *__restrict
                 for (uint32_t k = R + lane; k < ldy; k += 32) y[k] = 0.f;
                 acc = 0.f;
             }
-            cs.next(fptr, list, nlong);
+            cs.next(fibs, nlong);
         }
         if (g >= 0 && cr.live) {  // rows of stream group g
             const uint64_t mine = cr.first() + lane;
@@ -296,7 +351,7 @@ __global__ void __launch_bounds__(32) ttm_long_kernel(const uint64_t *__restrict
                                  : "memory");
                 }
             }
-            cr.next(fptr, list, nlong);
+            cr.next(fibs, nlong);
         }
         if (ci.live) {  // indices and values of stream group g + D
             const uint64_t mine = ci.first() + lane;
@@ -305,7 +360,7 @@ __global__ void __launch_bounds__(32) ttm_long_kernel(const uint64_t *__restrict
                 cp4(si + slot, sind + mine);
                 cp4(sx + slot, sval + mine);
             }
-            ci.next(fptr, list, nlong);
+            ci.next(fibs, nlong);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         __syncwarp();  // the slots read above are refilled in later iterations
@@ -633,7 +688,7 @@ int fiber_plan(ptiB200Tensor *t, uint32_t mode, bool sort, cudaStream_t s)
         PTI_TRY((exclusive_scan<uint64_t>(FiberHeadIn{a}, FiberOut{a}, n, tmp.as<uint64_t>(), &nfib, s)));
     }
     set_last_t<<<1, 1, 0, s>>>(P.fptr.as<uint64_t>(), nfib, n);
-    // fibers too long for one thread each (their order in the list is free:
+    // fibers too long for ttm_short_kernel (their order in the list is free:
     // every fiber is computed on its own)
     DevBuf cnt;
     PTI_CUDA(cnt.alloc(padded(16), s), mod);
@@ -650,8 +705,13 @@ int fiber_plan(ptiB200Tensor *t, uint32_t mode, bool sort, cudaStream_t s)
     P.nfib = nfib;
     P.nlong = nlong[0];
     P.nvlong = nlong[1];
-    // the fibers one thread takes, by length class (a stable sort of the
-    // classes, so fibers of one class stay in fiber order)
+    if (P.nlong) {
+        PTI_CUDA(P.long_fibs.alloc(padded(P.nlong * 16), s), mod);
+        pack_fibers_k<<<grid_t(P.nlong), 256, 0, s>>>(P.fptr.as<uint64_t>(), P.long_fibers.as<uint32_t>(), P.nlong,
+                                                      P.long_fibs.as<uint4>());
+    }
+    // the short fibers by length class (a stable sort of the classes, so
+    // fibers of one class stay in fiber order)
     P.nshort = nfib - P.nlong - P.nvlong;
     if (P.nshort) {
         DevBuf keys, order;
@@ -663,7 +723,7 @@ int fiber_plan(ptiB200Tensor *t, uint32_t mode, bool sort, cudaStream_t s)
                                                     order.as<uint32_t>());
         PTI_TRY(radix_sort_pairs(keys, order, nfib, 3, rs, s));
         PTI_CUDA(P.short_fibs.alloc(padded(P.nshort * 16), s), mod);
-        pack_short_k<<<grid_t(P.nshort), 256, 0, s>>>(P.fptr.as<uint64_t>(), order.as<uint32_t>(), P.nshort,
+        pack_fibers_k<<<grid_t(P.nshort), 256, 0, s>>>(P.fptr.as<uint64_t>(), order.as<uint32_t>(), P.nshort,
                                                        P.short_fibs.as<uint4>());
         PTI_CUDA(cudaStreamSynchronize(s), mod);
     }
@@ -692,8 +752,8 @@ int ttm_device(ptiB200Tensor *t, uint32_t mode, const float *U, uint32_t R, uint
     const uint32_t *si = P.sind.as<uint32_t>();
     const float *sv = P.sval.as<float>();
     const uint32_t nc4 = (R + 3) / 4;
-    // thread per short fiber: R <= 32, float4 rows (ldu, ldy multiples of 4
-    // and at least 4 * nc4, both arrays 16-byte aligned)
+    // lane groups of 4 columns a lane: R <= 32, float4 rows (ldu, ldy multiples
+    // of 4 and at least 4 * nc4, both arrays 16-byte aligned)
     const bool short_path = R <= 32 && ldu % 4 == 0 && ldy % 4 == 0 && ldu >= 4 * nc4 && ldy >= 4 * nc4 &&
                             reinterpret_cast<uintptr_t>(U) % 16 == 0 && reinterpret_cast<uintptr_t>(Y) % 16 == 0;
     uint64_t ngroup = P.nfib;
@@ -729,8 +789,7 @@ int ttm_device(ptiB200Tensor *t, uint32_t mode, const float *U, uint32_t R, uint
             PTI_CUDA(cudaFuncSetAttribute(ttm_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                      mod);
             const unsigned grid = (unsigned)std::min<uint64_t>(P.nlong, (uint64_t)sms * 8);
-            ttm_long_kernel<<<grid, 32, smem, s3>>>(fp, P.long_fibers.as<uint32_t>(), P.nlong, si, sv, U, ldu, R, W,
-                                                    Y, ldy);
+            ttm_long_kernel<<<grid, 32, smem, s3>>>(P.long_fibs.as<uint4>(), P.nlong, si, sv, U, ldu, R, W, Y, ldy);
             PTI_CUDA(cudaGetLastError(), mod);
             PTI_CUDA(cudaEventCreateWithFlags(&ev_l, cudaEventDisableTiming), mod);
             PTI_CUDA(cudaEventRecord(ev_l, s3), mod);
@@ -738,21 +797,19 @@ int ttm_device(ptiB200Tensor *t, uint32_t mode, const float *U, uint32_t R, uint
         joined = false;
     }
     if (short_path) {
-        // a thread per fiber and as many CTAs as that takes: CTAs finish in
-        // turn, so the long-fiber kernels beside this one find room
-        const unsigned g = (unsigned)std::max<uint64_t>(1, (P.nshort + 255) / 256);
+        // as many CTAs as the fibers take: CTAs finish in turn, so the
+        // long-fiber kernels beside this one find room
         const uint4 *sf = P.short_fibs.as<uint4>();
         const uint64_t ns = P.nshort;
-        if (ns) switch (nc4) {
-        case 1: ttm_short_kernel<1><<<g, 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R); break;
-        case 2: ttm_short_kernel<2><<<g, 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R); break;
-        case 3: ttm_short_kernel<3><<<g, 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R); break;
-        case 4: ttm_short_kernel<4><<<g, 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R); break;
-        case 5: ttm_short_kernel<5><<<g, 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R); break;
-        case 6: ttm_short_kernel<6><<<g, 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R); break;
-        case 7: ttm_short_kernel<7><<<g, 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R); break;
-        default: ttm_short_kernel<8><<<g, 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R); break;
-        }
+        auto go = [&](auto k, unsigned G) {
+            const unsigned per = 256 / G * kShortF;
+            k<<<(unsigned)((ns + per - 1) / per), 256, 0, s>>>(sf, ns, si, sv, U, ldu, Y, ldy, R);
+        };
+        if (!ns) {}
+        else if (nc4 <= 1) go(ttm_short_kernel<1>, 1);
+        else if (nc4 <= 2) go(ttm_short_kernel<2>, 2);
+        else if (nc4 <= 4) go(ttm_short_kernel<4>, 4);
+        else go(ttm_short_kernel<8>, 8);
         ngroup = 0;  // the long fibers are on the second stream
     }
     if (!joined) {  // `s` continues once the long fibers are done too
