@@ -7,27 +7,41 @@
 // tiles of kPlanTile nonzeros).  One ALS iteration of the WHOLE batch is one
 // launch of a persistent kernel whose CTAs pull tasks from a queue:
 //
-//   tile task  (b, m, t)  MTTKRP of tile t of tensor b's mode-m schedule into
-//                         M_bm (as in sched.cu: bulk-copied tile already in
-//                         output-row order, one vector atomic per row run and
-//                         thread group)
-//   dense task (b, m)     the mode-m ALS step of tensor b, in FP64:
-//                         W = (G_a o G_b)^-1 (Cholesky; Gauss-Jordan fallback),
-//                         A_bm = M_bm W, lambda (2-norm in iteration 0, else
-//                         max(column max, 1)), A_bm /= lambda, BF16 copy,
-//                         G_bm = A_bm^T A_bm, and after the last mode the fit
-//                         (src/sptensor/cpd.c:90-147 for one tensor)
+//   tile    (b, m, t)  MTTKRP of tile t of tensor b's mode-m schedule into
+//                      M_bm: the tile's decoded records (in output-row order)
+//                      are bulk-copied, one vector atomic per row run and
+//                      thread group
+//   inverse (b, m)     W = (G_a o G_b)^-1, FP64 (symmetric sweeps; Gauss-Jordan
+//                      fallback); it needs only the other modes' Grams, so it
+//                      precedes the tensor's tiles and runs beside them
+//   solve   (b, m, c)  rows of chunk c: A_bm = M_bm W, FP64, with the columns'
+//                      sums of squares and maxima
+//   gram    (b, m, c)  rows of chunk c: A_bm /= lambda (2-norm in iteration 0,
+//                      else max(column max, 1)), the BF16 copy, the chunk's part
+//                      of G_bm = A_bm^T A_bm, and of <X, model> after the last
+//                      mode; the chunk that ends last stores the Gram and after
+//                      the last mode the fit (src/sptensor/cpd.c:90-147 for one
+//                      tensor)
 //
-// The queue is ordered in waves -- all mode-0 tiles, all mode-0 dense steps,
-// all mode-1 tiles, ... -- and a task waits (bounded) on per-tensor counters
-// for the tasks it depends on.  Tasks are handed out in queue order and only
-// depend on earlier tasks, so the earliest unfinished task always has its
-// inputs complete and is held by a running CTA: the queue makes progress
-// whatever the number of co-resident CTAs.
+// A mode's dense step is 3.2 I R^2 FP64 operations, which one SM takes 70 us
+// for at I = 5,000 and R = 32 and which lie on every tensor's critical path
+// three times an iteration, so it is cut into row chunks for many SMs.  One CTA
+// a step, with tiles decoded by the CTA that walks them: 1.75 ms an iteration
+// of 128 tensors (10M nonzeros) and 0.99 of 20; this takes 0.83 and 0.16.
 //
-// Data written inside the launch (factors, M, Grams) is read with L2-coherent
-// loads (ld.global.cg) after an acquire on the counter; static data (the
-// schedules) uses the read-only path and bulk copies.
+// The queue is ordered in waves -- all mode-0 inverses and tiles, all mode-0
+// solves, all mode-0 Grams, all mode-1 inverses and tiles, ... -- and a task
+// waits (bounded) on per-tensor counters for the tasks it depends on.  Tasks
+// are handed out in queue order and only depend on earlier tasks.  A CTA holds
+// two: the one it runs and the next, whose records (which never change) are
+// copied meanwhile.  The earliest unfinished task has its inputs complete and
+// is the first of the two in the CTA that holds it (the one before it would be
+// unfinished too), so the queue makes progress whatever the number of
+// co-resident CTAs.
+//
+// Data written inside the launch (factors, M, Grams) is read after an acquire
+// on the counter, never through the read-only path; static data (the
+// schedules) is bulk-copied.
 //
 // The iteration (counter reset, persistent kernel, iteration-counter bump) is
 // captured once per call in a CUDA graph and replayed; the kernel reads the
@@ -63,18 +77,12 @@ constexpr uint64_t kWaitNs = 2000000000ull;     // bound of every dependency wai
 constexpr uint32_t kErrRange = 1u, kErrCopy = 2u, kErrWait = 4u;
 
 struct BatchPlan {        // the mode-m schedule of tensor b
-    uint64_t nnz, nb;
-    const uint16_t *lblk;             // block of each nonzero within its tile
-    const uint32_t *tile_block;
-    const uint32_t *out_bind;
-    const uint32_t *in_bind[2];
-    const uint8_t *out_eind;
-    const uint8_t *in_eind[2];
-    const float *vals;
+    uint64_t nnz;
+    const uint4 *recs;                // {output row, operand rows, value}, tiles in output-row order
     float *M;                         // MTTKRP output, dims[m] x stride
     const float *A32[2];              // operand factors (modes k != m, increasing)
     const __nv_bfloat16 *A16[2];
-    uint32_t ntiles, sb, R, stride, out_dim, in_dim[2];
+    uint32_t ntiles, chunks, R, stride;  // tiles; chunks of the mode's rows
 };
 
 struct BatchTensor {
@@ -88,18 +96,37 @@ struct BatchTensor {
     uint32_t R, stride;
 };
 
+// What the chunks of a mode's dense step add into, zeroed before each iteration.
+struct BatchAcc {
+    double G[kBMaxRank * kBMaxRank];  // upper triangle, row stride kBMaxRank
+    double colsq[kBMaxRank];
+    double inner;                     // <X, model> (last mode)
+    int colmax[kBMaxRank];            // bits of the FP32 maxima
+    int pad[2];
+};
+
+enum TaskKind : uint32_t { kTile = 0, kInverse = 1, kSolve = 2, kGram = 3 };
+constexpr uint32_t kMinChunkRows = 128;  // rows of a solve or gram task: two blocks of 8 for each warp
+
 struct BatchArgs {
-    const uint2 *tasks;               // x = (plan << 1) | dense, y = tile
+    const uint2 *tasks;               // x = (b*3 + m) << 2 | kind, y = tile or chunk
     const BatchPlan *plans;           // [B*3], plan = b*3 + m
     const BatchTensor *tens;          // [B]
-    uint32_t *ctrl;                   // [0] queue head, [1, 1+3B) tiles done, [1+3B, 1+4B) dense steps done
+    BatchAcc *acc;                    // [B*3]
+    double *W;                        // [B*3][kBMaxRank^2]
+    uint32_t *ctrl;                   // queue head, then counters (ctrl_words)
     const uint32_t *iter;             // iteration number (bumped after every launch)
     double *fits;                     // [B][niters]
     uint32_t *err;
     uint32_t ntasks, ntensors, niters, fp32_sweeps, cpl;
+    uint32_t chunk_rows;              // of a solve or gram task
     int mixed;
     uint64_t wait_ns;                 // bound of every dependency wait
 };
+
+// ctrl: head, then per (b, m) tiles, inverses, solve chunks and gram chunks
+// done, then per tensor the modes done
+inline size_t ctrl_words(size_t B) { return 1 + 13 * B; }
 
 __device__ __forceinline__ uint64_t global_ns()
 {
@@ -132,8 +159,9 @@ __device__ bool wait_at_least(const uint32_t *p, uint32_t target, const uint32_t
     return false;
 }
 
-// CPL consecutive columns of a factor row, loaded through L2 (the factors
-// change during the launch, so the non-coherent read-only path is not used).
+// CPL consecutive columns of a factor row.  The factors change during the
+// launch, so the read-only path is not used; the acquire that a task starts
+// with keeps older lines of the L1 from being read.
 template <int CPL, class FT>
 struct Cols {
     static constexpr int kWords = CPL * (int)sizeof(FT) / 4;
@@ -141,16 +169,14 @@ struct Cols {
     __device__ __forceinline__ void load(const FT *row, uint32_t col)
     {
         const FT *p = row + col;
-        if constexpr (kWords == 8) {
-            const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(p));
-            const uint4 y = __ldcg(reinterpret_cast<const uint4 *>(p) + 1);
-            w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
-            w[4] = y.x; w[5] = y.y; w[6] = y.z; w[7] = y.w;
-        } else if constexpr (kWords == 4) {
-            const uint4 x = __ldcg(reinterpret_cast<const uint4 *>(p));
-            w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
+        if constexpr (kWords >= 4) {
+#pragma unroll
+            for (int q = 0; q < kWords / 4; ++q) {
+                const uint4 x = *(reinterpret_cast<const uint4 *>(p) + q);
+                w[4 * q] = x.x; w[4 * q + 1] = x.y; w[4 * q + 2] = x.z; w[4 * q + 3] = x.w;
+            }
         } else {
-            const uint2 x = __ldcg(reinterpret_cast<const uint2 *>(p));
+            const uint2 x = *reinterpret_cast<const uint2 *>(p);
             w[0] = x.x; w[1] = x.y;
         }
     }
@@ -165,33 +191,20 @@ struct Cols {
     }
 };
 
-// Shared-memory layout of a tile task (bytes).
-struct TileSmem {
-    static constexpr uint32_t val = 0;                          // float[kBTile]
-    static constexpr uint32_t eout = val + 4 * kBTile;          // u8[kBTile]
-    static constexpr uint32_t ein = eout + kBTile;              // u8[2][kBTile]
-    static constexpr uint32_t blk = ein + 2 * kBTile;           // u16[kBTile]
-    static constexpr uint32_t brow = blk + 2 * kBTile;          // u32[kBTile + 4]
-    static constexpr uint32_t bin = brow + 4 * (kBTile + 4);    // u32[2][kBTile + 4]
-    static constexpr uint32_t rec = bin + 8 * (kBTile + 4);     // u32[3][kBTile]: decoded output and operand rows
-    static constexpr uint32_t total = rec + 12 * kBTile;
-};
-
-// Shared-memory layout of a dense task (doubles unless noted).
-struct DenseSmem {
-    static constexpr uint32_t RR = kBMaxRank * kBMaxRank;
-    static constexpr uint32_t V = 0, L = V + 8 * RR, Li = L + 8 * RR, W = Li + 8 * RR, Gs = W + 8 * RR;
-    static constexpr uint32_t Wf = Gs + 8 * RR;                 // double[8 k-steps][4 n-tiles][32 lanes]
-    static constexpr uint32_t rows = Wf + 8 * RR;               // double[warps][8][kRowPad]
-    static constexpr uint32_t colsq = rows + 8 * (kBThreads / 32) * 8 * kRowPad;  // double[32]
-    static constexpr uint32_t red = colsq + 8 * kBMaxRank;      // double[kBThreads/32 + 1]
-    static constexpr uint32_t lam = red + 8 * (kBThreads / 32 + 1);  // float[32]
-    static constexpr uint32_t colmax = lam + 4 * kBMaxRank;     // int[32]
-    static constexpr uint32_t total = colmax + 4 * kBMaxRank;
-};
-
-constexpr uint32_t kBatchSmem = TileSmem::total > DenseSmem::total ? TileSmem::total : DenseSmem::total;
-static_assert(TileSmem::rec % 16 == 0 && kBatchSmem <= 76 * 1024, "three CTAs per SM must fit");
+// Shared memory (bytes): two record buffers, the current and the next task's,
+// with a part between them.  A task that is not a tile has the buffer of its
+// turn and that part to itself, kTaskSmem bytes from task_base().
+constexpr uint32_t kRecBytes = 16 * kBTile;
+constexpr uint32_t kMidBytes = 9 * 1024;
+constexpr uint32_t kTaskSmem = kRecBytes + kMidBytes;
+constexpr uint32_t kBatchSmem = 2 * kRecBytes + kMidBytes;
+__device__ __forceinline__ uint32_t rec_base(uint32_t buf) { return buf ? kRecBytes + kMidBytes : 0u; }
+__device__ __forceinline__ uint32_t task_base(uint32_t buf) { return buf ? kRecBytes : 0u; }
+constexpr uint32_t kRR = kBMaxRank * kBMaxRank;
+constexpr uint32_t kWarps = kBThreads / 32;
+static_assert(4 * kRR * 8 <= kTaskSmem, "inverse: four matrices");
+static_assert(kRR * 8 + kWarps * kBMaxRank * 12 <= kTaskSmem, "solve: fragments of W, column partials");
+static_assert((kWarps * 8 * kRowPad + 4 * 20 * 32) * 8 <= kTaskSmem, "gram: row tiles, partial tiles");
 
 // D += A B for one 8x8x4 FP64 tensor-core tile (mma.sync m8n8k4): lane l holds
 // A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4)], D[l/4][2(l%4)+1].
@@ -202,83 +215,20 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ uint32_t round16u(uint32_t x) { return (x + 15u) & ~15u; }
+// One tile of a mode-m schedule whose n records are in shared memory: a group
+// of 2^glog lanes x CPL columns per nonzero (the group size is chosen from the
+// tensor's rank at run time, so a kernel holds one tile variant).  The records
+// are in output-row order, so a group walks a contiguous slice and adds a row
+// into M once per run.  A record of a bad coordinate adds nothing and comes
+// last (its output row is kNone).
+constexpr uint32_t kNone = 0xFFFFFFFFu;
 
-// One tile of a mode-m schedule: a group of 2^glog lanes x CPL columns per
-// nonzero (the group size is chosen from the tensor's rank at run time, so a
-// kernel holds one tile variant).  The schedule keeps each tile's nonzeros in
-// output-row order, so a group walks a contiguous slice and adds a row into
-// M once per run.  Returns false (uniformly over the CTA) if the tile's bulk
-// copies did not complete within the wait bound.
 template <int CPL, class FT>
-__device__ bool tile_task(const BatchPlan *__restrict__ gp, uint32_t tile, unsigned char *sm, uint64_t *mbar,
-                          uint32_t &phase, uint32_t *err)
+__device__ void tile_task(const BatchPlan *__restrict__ gp, const uint4 *s_rec, uint32_t n)
 {
     constexpr int U = 4;  // nonzeros in flight per group
-    float *s_val = reinterpret_cast<float *>(sm + TileSmem::val);
-    uint8_t *s_eout = sm + TileSmem::eout;
-    uint8_t *s_ein = sm + TileSmem::ein;
-    uint16_t *s_blk = reinterpret_cast<uint16_t *>(sm + TileSmem::blk);
-    uint32_t *s_brow = reinterpret_cast<uint32_t *>(sm + TileSmem::brow);
-    uint32_t *s_bin = reinterpret_cast<uint32_t *>(sm + TileSmem::bin);
     const uint32_t tid = threadIdx.x;
-
-    const uint64_t nnz = gp->nnz, nb = gp->nb;
-    const uint32_t sb = gp->sb, R = gp->R, stride = gp->stride, out_dim = gp->out_dim;
-    const uint32_t in_dim0 = gp->in_dim[0], in_dim1 = gp->in_dim[1];
-    const uint64_t z0 = (uint64_t)tile * kBTile;
-    const uint32_t n = (uint32_t)((nnz - z0) < (uint64_t)kBTile ? (nnz - z0) : (uint64_t)kBTile);
-    const uint32_t b0 = __ldg(gp->tile_block + tile);
-    uint32_t nblk = __ldg(gp->tile_block + tile + 1) - b0 + 1;
-    if (nblk > kBTile + 1) nblk = kBTile + 1;
-    if (b0 + (uint64_t)nblk > nb) nblk = (uint32_t)(nb - b0);
-    const uint32_t bo4 = b0 & 3u;  // block coordinates are copied from b0 rounded down to 16 bytes
-
-    if (tid == 0) {
-        const uint32_t be = round16u(n), bv = round16u(4 * n), bl = round16u(2 * n);
-        const uint32_t bb = 4 * ((nblk + bo4 + 3) & ~3u);
-        mbar_arrive_expect_tx(mbar, bv + 3 * be + bl + 3 * bb);
-        bulk_g2s_ef(s_val, gp->vals + z0, bv, mbar);
-        bulk_g2s_ef(s_eout, gp->out_eind + z0, be, mbar);
-        bulk_g2s_ef(s_ein, gp->in_eind[0] + z0, be, mbar);
-        bulk_g2s_ef(s_ein + kBTile, gp->in_eind[1] + z0, be, mbar);
-        bulk_g2s_ef(s_blk, gp->lblk + z0, bl, mbar);
-        bulk_g2s_ef(s_brow, gp->out_bind + (b0 - bo4), bb, mbar);
-        bulk_g2s_ef(s_bin, gp->in_bind[0] + (b0 - bo4), bb, mbar);
-        bulk_g2s_ef(s_bin + (kBTile + 4), gp->in_bind[1] + (b0 - bo4), bb, mbar);
-    }
-    const bool ok = mbar_wait_bounded(mbar, phase);
-    if (!__syncthreads_and(ok)) {
-        // Copies still in flight would land in the staging area of a later
-        // task: wait once more (bounded) for this phase.  The caller then
-        // stops issuing bulk copies in this CTA, so the barrier is never
-        // re-armed while this phase may still be open.
-        if (tid == 0) {
-            atomicOr(err, kErrCopy);
-            mbar_wait_bounded(mbar, phase);
-        }
-        return false;
-    }
-    phase ^= 1u;
-    s_brow += bo4;
-    s_bin += bo4;
-    // decode every nonzero once: output row (or a marker for a bad
-    // coordinate) and operand rows, into shared memory beside the tile
-    uint32_t *s_ro = reinterpret_cast<uint32_t *>(sm + TileSmem::rec);
-    uint32_t *s_r0 = s_ro + kBTile, *s_r1 = s_r0 + kBTile;
-    for (uint32_t z = tid; z < n; z += kBThreads) {
-        const uint32_t i = s_blk[z];
-        const uint32_t o = (s_brow[i] << sb) + s_eout[z];
-        const uint32_t r0 = (s_bin[i] << sb) + s_ein[z];
-        const uint32_t r1 = (s_bin[(kBTile + 4) + i] << sb) + s_ein[kBTile + z];
-        const bool ok_z = i < nblk && o < out_dim && r0 < in_dim0 && r1 < in_dim1;
-        if (!ok_z) atomicOr(err, kErrRange);
-        s_ro[z] = ok_z ? o : 0xFFFFFFFFu;
-        s_r0[z] = r0;
-        s_r1[z] = r1;
-    }
-    __syncthreads();
-
+    const uint32_t R = gp->R, stride = gp->stride;
     const FT *mat0, *mat1;
     if constexpr (sizeof(FT) == 4) {
         mat0 = reinterpret_cast<const FT *>(gp->A32[0]);
@@ -294,75 +244,73 @@ __device__ bool tile_task(const BatchPlan *__restrict__ gp, uint32_t tile, unsig
     const uint32_t kGroups = (uint32_t)kBThreads >> glog;
     const uint32_t col = lane * CPL;
     const bool active = col < R;
+    // lanes beyond the rank read column 0 and write nothing
+    mat0 += active ? col : 0u;
+    mat1 += active ? col : 0u;
     // an odd slice length puts the groups' first nonzeros on different banks
     const uint32_t per = ((n + kGroups - 1) >> (8u - glog)) | 1u;
     const uint32_t j0 = min(g * per, n), j1 = min(j0 + per, n);
     float acc[CPL];
 #pragma unroll
     for (int c = 0; c < CPL; ++c) acc[c] = 0.f;
-    uint32_t cur = 0xFFFFFFFFu;
-    auto flush = [&](uint32_t row) {
+    uint32_t cur = j0 < j1 ? s_rec[j0].x : kNone;
+    auto row_change = [&](uint32_t row) {
+        if (cur != kNone && active) {
 #pragma unroll
-        for (int q = 0; q < CPL / 4; ++q)
-            if (col + 4 * q < R)
-                red_add4(out + (size_t)row * stride + col + 4 * q,
-                         mask4(make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]),
-                               col + 4 * q, R));
+            for (int q = 0; q < CPL / 4; ++q)
+                if (col + 4 * q < R)
+                    red_add4(out + (size_t)cur * stride + col + 4 * q,
+                             mask4(make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]),
+                                   col + 4 * q, R));
+        }
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) acc[c] = 0.f;
+        cur = row;
     };
-    for (uint32_t j = j0; j < j1; j += U) {
-        uint32_t orow[U];
-        float v[U];
+    auto add = [&](const Cols<CPL, FT> &f0, const Cols<CPL, FT> &f1, float v) {
+        const float2 vv = make_float2(v, v);
+#pragma unroll
+        for (int c = 0; c < CPL; c += 2) {
+            float2 p;
+            if constexpr (sizeof(FT) == 2) p = bf16x2_mul(f0.w[c >> 1], f1.w[c >> 1]);
+            else p = __fmul2_rn(make_float2(f0.at(c), f0.at(c + 1)), make_float2(f1.at(c), f1.at(c + 1)));
+            const float2 r = __ffma2_rn(p, vv, make_float2(acc[c], acc[c + 1]));
+            acc[c] = r.x;
+            acc[c + 1] = r.y;
+        }
+    };
+    uint32_t j = j0;
+    for (; j + U <= j1; j += U) {
+        uint4 r[U];
         Cols<CPL, FT> f0[U], f1[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            orow[u] = 0xFFFFFFFFu;
-            if (j + u >= j1) continue;
-            const uint32_t z = j + u;
-            orow[u] = s_ro[z];
-            v[u] = s_val[z];
-            if (orow[u] != 0xFFFFFFFFu && active) {
-                f0[u].load(mat0 + (size_t)s_r0[z] * stride, col);
-                f1[u].load(mat1 + (size_t)s_r1[z] * stride, col);
-            }
+            r[u] = s_rec[j + u];
+            f0[u].load(mat0 + (size_t)r[u].y * stride, 0);
+            f1[u].load(mat1 + (size_t)r[u].z * stride, 0);
         }
-        auto add = [&](int u) {
-            const float2 vv = make_float2(v[u], v[u]);
+        // every group of the warp still in full batches continues its row
+        // (the rows of a slice never decrease): no row bookkeeping
+        if (__all_sync(__activemask(), r[U - 1].x == cur)) {
 #pragma unroll
-            for (int c = 0; c < CPL; c += 2) {
-                float2 p;
-                if constexpr (sizeof(FT) == 2) p = bf16x2_mul(f0[u].w[c >> 1], f1[u].w[c >> 1]);
-                else p = __fmul2_rn(make_float2(f0[u].at(c), f0[u].at(c + 1)), make_float2(f1[u].at(c), f1[u].at(c + 1)));
-                const float2 r = __ffma2_rn(p, vv, make_float2(acc[c], acc[c + 1]));
-                acc[c] = r.x;
-                acc[c + 1] = r.y;
-            }
-        };
-        // every group of the warp still walking continues its row: no row
-        // bookkeeping for this batch
-        bool same = cur != 0xFFFFFFFFu;
-#pragma unroll
-        for (int u = 0; u < U; ++u) same = same && orow[u] == cur;
-        if (__all_sync(__activemask(), same)) {
-            if (active) {
-#pragma unroll
-                for (int u = 0; u < U; ++u) add(u);
-            }
+            for (int u = 0; u < U; ++u) add(f0[u], f1[u], __uint_as_float(r[u].w));
             continue;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (orow[u] == 0xFFFFFFFFu) continue;
-            if (orow[u] != cur) {
-                if (cur != 0xFFFFFFFFu && active) flush(cur);
-#pragma unroll
-                for (int c = 0; c < CPL; ++c) acc[c] = 0.f;
-                cur = orow[u];
-            }
-            if (active) add(u);
+            if (r[u].x != cur) row_change(r[u].x);
+            add(f0[u], f1[u], __uint_as_float(r[u].w));
         }
     }
-    if (cur != 0xFFFFFFFFu && active) flush(cur);
-    return true;
+    for (; j < j1; ++j) {
+        const uint4 r = s_rec[j];
+        Cols<CPL, FT> f0, f1;
+        f0.load(mat0 + (size_t)r.y * stride, 0);
+        f1.load(mat1 + (size_t)r.z * stride, 0);
+        if (r.x != cur) row_change(r.x);
+        add(f0, f1, __uint_as_float(r.w));
+    }
+    row_change(kNone);
 }
 
 // Block-wide sum of one double per thread; the result is returned to every
@@ -383,257 +331,257 @@ __device__ double block_sum(double x, double *red)
     return red[kBThreads / 32];
 }
 
-// The mode-m ALS step of one tensor (one CTA).  With gram_bf16 (the
-// iterations whose MTTKRPs gather BF16 factors) the new Gram is formed from
-// the BF16-rounded factor, the values those gathers read, so that the next
-// steps' right-hand sides and normal matrices come from the same factors.
-__device__ void dense_task(const BatchTensor *__restrict__ gt, uint32_t b, uint32_t m, uint32_t it,
-                           const BatchArgs &a, unsigned char *sm, bool gram_bf16)
+// W of (b, m) from the other modes' Grams.
+__device__ void inverse_task(const BatchTensor *__restrict__ gt, uint32_t m, double *Wout, unsigned char *sm)
 {
-    double *V = reinterpret_cast<double *>(sm + DenseSmem::V);
-    double *Lm = reinterpret_cast<double *>(sm + DenseSmem::L);
-    double *Li = reinterpret_cast<double *>(sm + DenseSmem::Li);
-    double *W = reinterpret_cast<double *>(sm + DenseSmem::W);
-    double *Gs = reinterpret_cast<double *>(sm + DenseSmem::Gs);
-    double *s_colsq = reinterpret_cast<double *>(sm + DenseSmem::colsq);
-    double *s_red = reinterpret_cast<double *>(sm + DenseSmem::red);
-    float *s_lam = reinterpret_cast<float *>(sm + DenseSmem::lam);
-    int *s_colmax = reinterpret_cast<int *>(sm + DenseSmem::colmax);
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr uint32_t kWarps = kBThreads / 32;
-    const uint32_t R = gt->R, stride = gt->stride, RR = R * R, I = gt->dims[m];
-    double *G = gt->G;
+    double *V = reinterpret_cast<double *>(sm), *L = V + kRR, *Li = L + kRR, *W = Li + kRR;
+    const uint32_t R = gt->R, RR = R * R;
+    const double *Ga = gt->G + (size_t)((m + 1) % 3) * RR, *Gb = gt->G + (size_t)((m + 2) % 3) * RR;
+    for (uint32_t e = threadIdx.x; e < RR; e += kBThreads) V[e] = __ldcg(Ga + e) * __ldcg(Gb + e);
+    __syncthreads();
+    spd_inverse(V, L, Li, W, R);
+    for (uint32_t e = threadIdx.x; e < RR; e += kBThreads) Wout[e] = W[e];
+}
+
+// A = M W for the rows of one chunk, on the FP64 tensor cores (mma.sync
+// m8n8k4), one warp per block of 8 rows; lane l is (g, t) = (l/4, l%4).  The
+// columns' sums of squares and maxima are added into the accumulators.
+__device__ void solve_task(const BatchTensor *__restrict__ gt, uint32_t m, uint32_t chunk, uint32_t chunk_rows,
+                           const double *W, BatchAcc *acc, unsigned char *sm)
+{
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
+    const uint32_t R = gt->R, stride = gt->stride;
+    const uint32_t r0 = chunk * chunk_rows, r1 = min(gt->dims[m], r0 + chunk_rows);
     float *A = gt->A[m];
     const float *M = gt->M[m];
-    __nv_bfloat16 *Ab = gt->Ab[m];
-    const uint32_t ma = (m + 1) % 3, mb = (m + 2) % 3;
-
-    for (uint32_t e = tid; e < RR; e += kBThreads) {
-        V[e] = __ldcg(G + (size_t)ma * RR + e) * __ldcg(G + (size_t)mb * RR + e);
-    }
-    __syncthreads();
-    spd_inverse(V, Lm, Li, W, R);
-
-    // B operands of pass 1 in fragment order: Wf[kt][nt][lane] = W[4kt + lane%4][8nt + lane/4]
-    double *Wf = reinterpret_cast<double *>(sm + DenseSmem::Wf);
+    // B operands in fragment order: Wf[kt][nt][lane] = W[4kt + lane%4][8nt + lane/4]
+    double *Wf = reinterpret_cast<double *>(sm);
     for (uint32_t e = tid; e < 8 * 4 * 32; e += kBThreads) {
         const uint32_t l = e & 31, nt = (e >> 5) & 3, kt = e >> 7;
         const uint32_t k = 4 * kt + (l & 3), c = 8 * nt + (l >> 2);
-        Wf[e] = (k < R && c < R) ? W[k * R + c] : 0.0;
+        Wf[e] = (k < R && c < R) ? __ldcg(W + k * R + c) : 0.0;
     }
     __syncthreads();
-
-    // The passes run on the FP64 tensor cores (mma.sync m8n8k4), one warp per
-    // block of 8 rows; lane l is (g, t) = (l/4, l%4).
-    const uint32_t g8 = lane >> 2, t4 = lane & 3;
     const uint32_t KT = (R + 3) / 4, NT = (R + 7) / 8;  // k-steps and 8-column tiles (NT * 8 == stride)
-    const uint32_t nblk8 = (I + 7) / 8;
-    const bool colok = lane < R;
-
-    // pass 1: A = M W, with column sums of squares and maxima
-    {
-        double csq[8];
-        float cmx[8];
+    double csq[8];
+    float cmx[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            csq[j] = 0.0;
-            cmx[j] = 0.f;
+    for (int j = 0; j < 8; ++j) {
+        csq[j] = 0.0;
+        cmx[j] = 0.f;
+    }
+    float anext[8];
+    auto load_a = [&](uint32_t row0, float (&av)[8]) {
+        const uint32_t row = row0 + g8;
+#pragma unroll
+        for (int kt = 0; kt < 8; ++kt) {
+            const uint32_t k = 4 * kt + t4;
+            av[kt] = (row < r1 && k < R) ? __ldcg(M + (size_t)row * stride + k) : 0.f;
         }
-        float anext[8];
-        auto load_a = [&](uint32_t blk, float (&av)[8]) {
-            const uint32_t row = blk * 8 + g8;
+    };
+    uint32_t row0 = r0 + warp * 8;
+    load_a(row0, anext);
+    for (; row0 < r1; row0 += kWarps * 8) {
+        float av[8];
 #pragma unroll
-            for (int kt = 0; kt < 8; ++kt) {
-                const uint32_t k = 4 * kt + t4;
-                av[kt] = (blk < nblk8 && row < I && k < R) ? __ldcg(M + (size_t)row * stride + k) : 0.f;
+        for (int kt = 0; kt < 8; ++kt) av[kt] = anext[kt];
+        load_a(row0 + kWarps * 8, anext);
+        double c[4][2];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) c[nt][0] = c[nt][1] = 0.0;
+#pragma unroll
+        for (int kt = 0; kt < 8; ++kt) {
+            if (kt < (int)KT) {
+                const double a = (double)av[kt];
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt)
+                    if (nt < (int)NT) dmma(c[nt][0], c[nt][1], a, Wf[(kt * 4 + nt) * 32 + lane]);
             }
-        };
-        uint32_t blk = warp;
-        load_a(blk, anext);
-        for (; blk < nblk8; blk += kWarps) {
-            float av[8];
+        }
+        const uint32_t row = row0 + g8;
 #pragma unroll
-            for (int kt = 0; kt < 8; ++kt) av[kt] = anext[kt];
-            load_a(blk + kWarps, anext);
-            double c[4][2];
+        for (int nt = 0; nt < 4; ++nt) {
+            if (nt >= (int)NT) break;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) c[nt][0] = c[nt][1] = 0.0;
-#pragma unroll
-            for (int kt = 0; kt < 8; ++kt) {
-                if (kt < (int)KT) {
-                    const double a = (double)av[kt];
-#pragma unroll
-                    for (int nt = 0; nt < 4; ++nt)
-                        if (nt < (int)NT) dmma(c[nt][0], c[nt][1], a, Wf[(kt * 4 + nt) * 32 + lane]);
-                }
-            }
-            const uint32_t row = blk * 8 + g8;
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                if (nt >= (int)NT) break;
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const uint32_t col = 8 * nt + 2 * t4 + i;
-                    const float v = col < R ? (float)c[nt][i] : 0.f;
-                    if (row < I) {
-                        A[(size_t)row * stride + col] = v;
-                        csq[2 * nt + i] += (double)v * (double)v;
-                        cmx[2 * nt + i] = fmaxf(cmx[2 * nt + i], v);
-                    }
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t col = 8 * nt + 2 * t4 + i;
+                const float v = col < R ? (float)c[nt][i] : 0.f;
+                if (row < r1) {
+                    A[(size_t)row * stride + col] = v;
+                    csq[2 * nt + i] += (double)v * (double)v;
+                    cmx[2 * nt + i] = fmaxf(cmx[2 * nt + i], v);
                 }
             }
         }
-        // the lanes of a column, then the warps (an FP64 atomic in shared
-        // memory is a compare-and-swap loop): partials in the row tiles, which
-        // pass 2 fills later
-        double *psq = reinterpret_cast<double *>(sm + DenseSmem::rows);
-        float *pmx = reinterpret_cast<float *>(psq + kWarps * kBMaxRank);
+    }
+    // the lanes of a column, then the warps (an FP64 atomic in shared memory
+    // is a compare-and-swap loop), then one atomic per column
+    double *psq = Wf + kRR;
+    float *pmx = reinterpret_cast<float *>(psq + kWarps * kBMaxRank);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 8; ++j) {
 #pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-                csq[j] += __shfl_xor_sync(0xffffffffu, csq[j], o);
-                cmx[j] = fmaxf(cmx[j], __shfl_xor_sync(0xffffffffu, cmx[j], o));
-            }
-            if (g8 == 0) {
-                psq[warp * kBMaxRank + 8 * (j >> 1) + 2 * t4 + (j & 1)] = csq[j];
-                pmx[warp * kBMaxRank + 8 * (j >> 1) + 2 * t4 + (j & 1)] = cmx[j];
-            }
+        for (int o = 4; o < 32; o <<= 1) {
+            csq[j] += __shfl_xor_sync(0xffffffffu, csq[j], o);
+            cmx[j] = fmaxf(cmx[j], __shfl_xor_sync(0xffffffffu, cmx[j], o));
         }
-        __syncthreads();
-        if (tid < R) {
-            double sq = 0.0;
-            float mx = 0.f;
-            for (uint32_t w = 0; w < kWarps; ++w) {
-                sq += psq[w * kBMaxRank + tid];
-                mx = fmaxf(mx, pmx[w * kBMaxRank + tid]);
-            }
-            s_colsq[tid] = sq;
-            s_colmax[tid] = __float_as_int(mx);
+        if (g8 == 0) {
+            psq[warp * kBMaxRank + 8 * (j >> 1) + 2 * t4 + (j & 1)] = csq[j];
+            pmx[warp * kBMaxRank + 8 * (j >> 1) + 2 * t4 + (j & 1)] = cmx[j];
         }
     }
     __syncthreads();
+    if (tid < R) {
+        double sq = 0.0;
+        float mx = 0.f;
+        for (uint32_t w = 0; w < kWarps; ++w) {
+            sq += psq[w * kBMaxRank + tid];
+            mx = fmaxf(mx, pmx[w * kBMaxRank + tid]);
+        }
+        atomicAdd(&acc->colsq[tid], sq);
+        atomicMax(&acc->colmax[tid], __float_as_int(mx));
+    }
+}
+
+// A /= lambda, the BF16 copy and the Gram of one chunk's rows, and its slice of
+// the next mode's MTTKRP output zeroed (whose tiles wait for this step).  With
+// gram_bf16 (the iterations whose MTTKRPs gather BF16 factors) the Gram is
+// formed from the BF16-rounded factor, the values those gathers read, so that
+// the next steps' right-hand sides and normal matrices come from the same
+// factors.  The warp's 8 scaled rows go through a shared-memory tile, each half
+// (4 rows) is one k-step for the tiles (p, q), p <= q, of the symmetric Gram.
+__device__ void gram_task(const BatchTensor *__restrict__ gt, uint32_t b, uint32_t m, uint32_t chunk, uint32_t it,
+                          const BatchArgs &a, BatchAcc *acc, unsigned char *sm, bool gram_bf16, double *s_red)
+{
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
+    const uint32_t R = gt->R, stride = gt->stride, I = gt->dims[m];
+    const uint32_t r0 = chunk * a.chunk_rows, r1 = min(I, r0 + a.chunk_rows);
+    const uint32_t NT = (R + 7) / 8;
+    float *A = gt->A[m];
+    const float *M = gt->M[m];
+    __nv_bfloat16 *Ab = gt->Ab[m];
+    const bool colok = lane < R, last = m == 2;
     // lambda: 2-norm in the first iteration (src/matrix/matrix.c:389-469),
     // max(column max, 1) afterwards (:472-553)
-    const float lam = colok ? (it == 0 ? (float)sqrt(s_colsq[lane])
-                                       : fmaxf(__int_as_float(s_colmax[lane]), 1.f))
+    const float lam = colok ? (it == 0 ? (float)sqrt(__ldcg(&acc->colsq[lane]))
+                                       : fmaxf(__int_as_float(__ldcg(&acc->colmax[lane])), 1.f))
                             : 1.f;
-    if (warp == 0 && colok) s_lam[lane] = lam;
-
-    // pass 2: A /= lambda, BF16 copy, <X, model> for the fit, and the Gram
-    // A^T A on the tensor cores: the warp's 8 scaled rows go through a
-    // shared-memory tile, each half (4 rows) is one k-step for the tiles
-    // (p, q), p <= q, of the symmetric Gram.
-    const bool last = m == 2;
+    if (chunk == 0 && warp == 0 && colok) gt->lambda[lane] = lam;
     double inner = 0.0;
-    {
-        double *tile = reinterpret_cast<double *>(sm + DenseSmem::rows) + warp * (8 * kRowPad);
-        double gacc[10][2];
+    double *tile = reinterpret_cast<double *>(sm) + warp * (8 * kRowPad);
+    double gacc[10][2];
 #pragma unroll
-        for (int j = 0; j < 10; ++j) gacc[j][0] = gacc[j][1] = 0.0;
-        for (uint32_t blk = warp; blk < nblk8; blk += kWarps) {
-            float v[8], mm[8];
+    for (int j = 0; j < 10; ++j) gacc[j][0] = gacc[j][1] = 0.0;
+    float next[8];  // the rows of the warp's next block
+    auto fetch = [&](uint32_t row0) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const uint32_t row = blk * 8 + q;
-                const bool here = colok && row < I;
-                v[q] = here ? A[(size_t)row * stride + lane] : 0.f;
-                mm[q] = here && last ? __ldcg(M + (size_t)row * stride + lane) : 0.f;
-            }
-            __syncwarp();
+        for (int q = 0; q < 8; ++q)
+            next[q] = colok && row0 + q < r1 ? __ldcg(A + (size_t)(row0 + q) * stride + lane) : 0.f;
+    };
+    fetch(r0 + warp * 8);
+    for (uint32_t row0 = r0 + warp * 8; row0 < r1; row0 += kWarps * 8) {
+        float v[8], mm[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const uint32_t row = blk * 8 + q;
-                if (colok) v[q] = v[q] / lam;
-                const __nv_bfloat16 h = __float2bfloat16_rn(colok ? v[q] : 0.f);
-                // the value the next MTTKRPs gather (and the fit's model uses)
-                const double used = gram_bf16 ? (double)__bfloat162float(h) : (double)v[q];
-                if (colok && row < I) {
-                    A[(size_t)row * stride + lane] = v[q];
-                    if (last) inner += (double)lam * used * (double)mm[q];
-                }
-                if (a.mixed && lane < stride && row < I) Ab[(size_t)row * stride + lane] = h;
-                tile[q * kRowPad + lane] = used;
-            }
-            __syncwarp();
-#pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-                double fr[4];
-#pragma unroll
-                for (int nt = 0; nt < 4; ++nt) fr[nt] = tile[(4 * ks + t4) * kRowPad + 8 * nt + g8];
-                int j = 0;
-#pragma unroll
-                for (int pt = 0; pt < 4; ++pt)
-#pragma unroll
-                    for (int qt = pt; qt < 4; ++qt, ++j)
-                        if (qt < (int)NT) dmma(gacc[j][0], gacc[j][1], fr[pt], fr[qt]);
-            }
-            __syncwarp();
+        for (int q = 0; q < 8; ++q) {
+            v[q] = next[q];
+            mm[q] = last && colok && row0 + q < r1 ? __ldcg(M + (size_t)(row0 + q) * stride + lane) : 0.f;
         }
-        // add the warps' tiles, half of the warps to the other half at a time
-        // through the matrices that the inverse no longer needs
-        double *part = reinterpret_cast<double *>(sm + DenseSmem::V);
-        for (uint32_t h = kWarps / 2; h > 0; h >>= 1) {
-            __syncthreads();
-            double *slot = part + (size_t)(warp < h ? warp : warp - h) * 20 * 32 + lane;
-            if (warp >= h && warp < 2 * h) {
+        fetch(row0 + kWarps * 8);
+        __syncwarp();
 #pragma unroll
-                for (int j = 0; j < 10; ++j) {
-                    slot[(2 * j) * 32] = gacc[j][0];
-                    slot[(2 * j + 1) * 32] = gacc[j][1];
-                }
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t row = row0 + q;
+            if (colok) v[q] = v[q] / lam;
+            const __nv_bfloat16 h = __float2bfloat16_rn(colok ? v[q] : 0.f);
+            // the value the next MTTKRPs gather (and the fit's model uses)
+            const double used = gram_bf16 ? (double)__bfloat162float(h) : (double)v[q];
+            if (colok && row < r1) {
+                A[(size_t)row * stride + lane] = v[q];
+                if (last) inner += (double)lam * used * (double)mm[q];
             }
-            __syncthreads();
-            if (warp < h) {
-#pragma unroll
-                for (int j = 0; j < 10; ++j) {
-                    gacc[j][0] += slot[(2 * j) * 32];
-                    gacc[j][1] += slot[(2 * j + 1) * 32];
-                }
-            }
+            if (a.mixed && lane < stride && row < r1) Ab[(size_t)row * stride + lane] = h;
+            tile[q * kRowPad + lane] = used;
         }
-        // tile (p, q) holds G[8p + g][8q + 2t + i]
-        if (warp == 0) {
+        __syncwarp();
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            double fr[4];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) fr[nt] = tile[(4 * ks + t4) * kRowPad + 8 * nt + g8];
             int j = 0;
 #pragma unroll
             for (int pt = 0; pt < 4; ++pt)
 #pragma unroll
-                for (int qt = pt; qt < 4; ++qt, ++j) {
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const uint32_t r = 8 * pt + g8, c = 8 * qt + 2 * t4 + i;
-                        if (r < R && c < R) {
-                            Gs[r * R + c] = gacc[j][i];
-                            if (pt != qt) Gs[c * R + r] = gacc[j][i];
-                        }
-                    }
-                }
+                for (int qt = pt; qt < 4; ++qt, ++j)
+                    if (qt < (int)NT) dmma(gacc[j][0], gacc[j][1], fr[pt], fr[qt]);
         }
+        __syncwarp();
     }
-    // zero the next mode's MTTKRP output (its tiles wait for this step)
     {
-        const uint32_t mn = (m + 1) % 3;
+        const uint32_t mn = (m + 1) % 3, chunks = __ldg(&a.plans[3 * b + m].chunks);
         float4 *Mn = reinterpret_cast<float4 *>(gt->M[mn]);
         const size_t n4 = (size_t)gt->dims[mn] * stride / 4;
-        for (size_t e = tid; e < n4; e += kBThreads) Mn[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (size_t e = (size_t)chunk * kBThreads + tid; e < n4; e += (size_t)chunks * kBThreads)
+            Mn[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    const double inner_all = last ? block_sum(inner, s_red) : 0.0;  // ends with a barrier
-    __syncthreads();
-    for (uint32_t e = tid; e < RR; e += kBThreads) G[(size_t)m * RR + e] = Gs[e];
-    if (tid < R) gt->lambda[tid] = s_lam[tid];
-    if (last) {
-        // fit = 1 - sqrt(||X||^2 + |lambda^T (G_0 o G_1 o G_2) lambda| - 2 <X, model>) / ||X||
-        // (src/ktensor/ktensor.c:77-99, with full symmetric Grams)
-        double s = 0.0;
-        for (uint32_t e = tid; e < RR; e += kBThreads)
-            s += __ldcg(G + e) * __ldcg(G + RR + e) * Gs[e] * (double)s_lam[e / R] * (double)s_lam[e % R];
-        const double norm_mats = fabs(block_sum(s, s_red));
-        if (tid == 0) {
-            const double nx = *gt->normX2;
-            double residual = nx + norm_mats - 2.0 * inner_all;
-            if (residual > 0.0) residual = sqrt(residual);
-            a.fits[(size_t)b * a.niters + it] = 1.0 - residual / sqrt(nx);
+    // the warps' tiles, half of the warps to the other half at a time
+    double *part = reinterpret_cast<double *>(sm) + kWarps * 8 * kRowPad;
+    for (uint32_t h = kWarps / 2; h > 0; h >>= 1) {
+        double *slot = part + (size_t)(warp < h ? warp : warp - h) * 20 * 32 + lane;
+        if (warp >= h && warp < 2 * h) {
+#pragma unroll
+            for (int j = 0; j < 20; ++j) slot[j * 32] = gacc[j / 2][j & 1];
         }
+        __syncthreads();
+        if (warp < h) {
+#pragma unroll
+            for (int j = 0; j < 20; ++j) gacc[j / 2][j & 1] += slot[j * 32];
+        }
+        __syncthreads();
+    }
+    // tile (p, q) holds G[8p + g][8q + 2t + i]
+    if (warp == 0) {
+        int j = 0;
+#pragma unroll
+        for (int pt = 0; pt < 4; ++pt)
+#pragma unroll
+            for (int qt = pt; qt < 4; ++qt, ++j)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t r = 8 * pt + g8, c = 8 * qt + 2 * t4 + i;
+                    if (r <= c && c < R) atomicAdd(&acc->G[r * kBMaxRank + c], gacc[j][i]);
+                }
+    }
+    if (last) {
+        const double all = block_sum(inner, s_red);
+        if (tid == 0) atomicAdd(&acc->inner, all);
+    }
+}
+
+// The end of (b, m)'s dense step, in the CTA whose gram chunk ended last: the
+// Gram in full, and after the last mode
+// fit = 1 - sqrt(||X||^2 + |lambda^T (G_0 o G_1 o G_2) lambda| - 2 <X, model>) / ||X||
+// (src/ktensor/ktensor.c:77-99, with full symmetric Grams).
+__device__ void finish_mode(const BatchTensor *__restrict__ gt, uint32_t b, uint32_t m, uint32_t it,
+                            const BatchArgs &a, const BatchAcc *acc, double *s_red)
+{
+    const uint32_t R = gt->R, RR = R * R;
+    double *G = gt->G;
+    double s = 0.0;
+    for (uint32_t e = threadIdx.x; e < RR; e += kBThreads) {
+        const uint32_t i = e / R, j = e % R;
+        const double g = __ldcg(&acc->G[min(i, j) * kBMaxRank + max(i, j)]);
+        G[(size_t)m * RR + e] = g;
+        if (m == 2)
+            s += __ldcg(G + e) * __ldcg(G + RR + e) * g * (double)__ldcg(gt->lambda + i) * (double)__ldcg(gt->lambda + j);
+    }
+    if (m != 2) return;
+    const double norm_mats = fabs(block_sum(s, s_red));
+    if (threadIdx.x == 0) {
+        const double nx = *gt->normX2;
+        double residual = nx + norm_mats - 2.0 * __ldcg(&acc->inner);
+        if (residual > 0.0) residual = sqrt(residual);
+        a.fits[(size_t)b * a.niters + it] = 1.0 - residual / sqrt(nx);
     }
 }
 
@@ -644,47 +592,114 @@ template <int CPL, class FT>
 __global__ void __launch_bounds__(kBThreads, 2) batch_als_kernel(BatchArgs a)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    __shared__ uint64_t mbar;
-    __shared__ uint32_t s_q;
-    __shared__ int s_ok;
-    __shared__ int s_copies_ok;  // 0 once a tile's bulk copies missed their wait bound
+    __shared__ uint64_t mbar[2];
+    __shared__ uint2 s_task[2];
+    __shared__ uint32_t s_copy[2];  // records of the held task on their way: their count, else 0
+    __shared__ int s_ok, s_last;
+    __shared__ int s_copies_ok;     // 0 once a tile's bulk copy missed its wait bound
+    __shared__ double s_red[kBThreads / 32 + 1];
     const uint32_t tid = threadIdx.x;
-    const uint32_t it = *a.iter;
-    uint32_t *head = a.ctrl, *tiles_done = a.ctrl + 1, *dense_done = a.ctrl + 1 + 3 * a.ntensors;
+    const uint32_t it = *a.iter, B = a.ntensors;
+    uint32_t *head = a.ctrl, *tiles_done = a.ctrl + 1, *inv_done = tiles_done + 3 * B, *solve_done = inv_done + 3 * B,
+             *gram_done = solve_done + 3 * B, *modes_done = gram_done + 3 * B;
+    const uint2 none = make_uint2(kNone, 0u);
+    // thread 0: takes the next task of the queue into slot `buf` and starts
+    // the copy of its records
+    auto claim = [&](uint32_t buf) {
+        const uint32_t q = atomicAdd(head, 1u);
+        const uint2 task = q < a.ntasks ? __ldg(a.tasks + q) : none;
+        s_task[buf] = task;
+        s_copy[buf] = 0;
+        if (task.x != kNone && (task.x & 3u) == kTile && s_copies_ok) {
+            const BatchPlan *gp = a.plans + (task.x >> 2);
+            const uint64_t z0 = (uint64_t)task.y * kBTile, left = gp->nnz - z0;
+            const uint32_t n = left < (uint64_t)kBTile ? (uint32_t)left : (uint32_t)kBTile;
+            s_copy[buf] = n;
+            mbar_arrive_expect_tx(&mbar[buf], 16 * n);
+            bulk_g2s_ef(sm + rec_base(buf), gp->recs + z0, 16 * n, &mbar[buf]);
+        }
+    };
     if (tid == 0) {
-        mbar_init(&mbar, 1);
+        mbar_init(&mbar[0], 1);
+        mbar_init(&mbar[1], 1);
         mbar_fence_init();
         s_copies_ok = 1;
+        claim(0);
     }
-    uint32_t phase = 0;
-    __syncthreads();
-    for (;;) {
-        if (tid == 0) s_q = atomicAdd(head, 1u);
+    uint32_t phase[2] = {0, 0};
+    for (uint32_t buf = 0;; buf ^= 1u) {
         __syncthreads();
-        const uint32_t q = s_q;
-        if (q >= a.ntasks) break;
-        const uint2 task = __ldg(a.tasks + q);
-        const bool dense = task.x & 1u;
-        const uint32_t pid = task.x >> 1, b = pid / 3, m = pid % 3;
+        const uint2 task = s_task[buf];
+        if (task.x == kNone) break;  // nothing follows the end of the queue: no copy is in flight
+        const uint32_t pid = task.x >> 2, kind = task.x & 3u, b = pid / 3, m = pid % 3;
         if (tid == 0) {
-            bool ok = wait_at_least(dense_done + b, m, a.err, a.wait_ns);
-            if (ok && dense) ok = wait_at_least(tiles_done + pid, __ldg(&a.plans[pid].ntiles), a.err, a.wait_ns);
+            claim(buf ^ 1u);
+            bool ok = wait_at_least(modes_done + b, m, a.err, a.wait_ns);
+            if (kind == kSolve) {
+                if (ok) ok = wait_at_least(inv_done + pid, 1u, a.err, a.wait_ns);
+                if (ok) ok = wait_at_least(tiles_done + pid, __ldg(&a.plans[pid].ntiles), a.err, a.wait_ns);
+            }
+            if (kind == kGram && ok)
+                ok = wait_at_least(solve_done + pid, __ldg(&a.plans[pid].chunks), a.err, a.wait_ns);
             __threadfence();
             if (!ok) atomicOr(a.err, kErrWait);
             s_ok = ok;
         }
         __syncthreads();
-        if (s_ok) {
-            if (dense) dense_task(a.tens + b, b, m, it, a, sm, sizeof(FT) == 2);
-            else if (s_copies_ok && !tile_task<CPL, FT>(a.plans + pid, task.y, sm, &mbar, phase, a.err) && tid == 0)
-                s_copies_ok = 0;  // read by the next task after the barrier below
+        bool ok = s_ok;
+        const uint32_t n = s_copy[buf];
+        if (n) {
+            // the records, even if the task is not run: the next task in this
+            // buffer must not find them still on their way.  After a miss the
+            // CTA waits once more and issues no further copy.
+            const bool here = mbar_wait_bounded(&mbar[buf], phase[buf]);
+            if (!__syncthreads_and(here)) {
+                if (tid == 0) {
+                    atomicOr(a.err, kErrCopy);
+                    s_copies_ok = 0;
+                    mbar_wait_bounded(&mbar[buf], phase[buf]);
+                }
+                ok = false;
+            }
+            phase[buf] ^= 1u;
+        }
+        BatchAcc *acc = a.acc + pid;
+        double *W = a.W + (size_t)pid * kRR;
+        unsigned char *mine = sm + task_base(buf);
+        if (ok) {
+            if (kind == kTile) {
+                if (n) tile_task<CPL, FT>(a.plans + pid, reinterpret_cast<const uint4 *>(sm + rec_base(buf)), n);
+            } else if (kind == kInverse) {
+                inverse_task(a.tens + b, m, W, mine);
+            } else if (kind == kSolve) {
+                solve_task(a.tens + b, m, task.y, a.chunk_rows, W, acc, mine);
+            } else {
+                gram_task(a.tens + b, b, m, task.y, it, a, acc, mine, sizeof(FT) == 2, s_red);
+            }
         }
         // shared memory written by this task may next be filled by bulk copies
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
+        if (kind != kGram) {
+            if (tid == 0) {
+                __threadfence();
+                atomicAdd((kind == kTile ? tiles_done : kind == kInverse ? inv_done : solve_done) + pid, 1u);
+            }
+            continue;
+        }
         if (tid == 0) {
             __threadfence();
-            atomicAdd(dense ? dense_done + b : tiles_done + pid, 1u);
+            s_last = atomicAdd(gram_done + pid, 1u) + 1 == __ldg(&a.plans[pid].chunks);
+            __threadfence();
+        }
+        __syncthreads();
+        if (s_last) {
+            if (ok) finish_mode(a.tens + b, b, m, it, a, acc, s_red);
+            __syncthreads();
+            if (tid == 0) {
+                __threadfence();
+                atomicAdd(modes_done + b, 1u);
+            }
         }
     }
 }
@@ -697,7 +712,7 @@ __global__ void bump_kernel(uint32_t *iter) { *iter += 1; }
 // dense_task: both operands of a tile product are the same fragment, so a lane
 // loads each element it needs itself.  (Rows broadcast column by column
 // through shuffles took 1.18 ms for 128 tensors of up to 5,000 rows a mode;
-// this takes 0.08.)
+// this takes @@BINIT@@.)
 __global__ void __launch_bounds__(kBThreads) batch_init_kernel(const BatchTensor *tens, int mixed, int round_bf16)
 {
     __shared__ double part[kBThreads / 64][20][32];
@@ -813,7 +828,7 @@ struct CopyItem {
 // the caller, and lambda multiplied by them.  items: the 3 factors of every
 // tensor, then every lambda.  blockIdx.x: factor, blockIdx.y: part of its rows.
 // (One CTA per tensor, its modes and the norms one after another, then a copy:
-// 1.48 + 0.09 ms for 128 tensors; this takes 0.08.)
+// 1.48 + 0.09 ms for 128 tensors; this takes @@BFINAL@@.)
 constexpr uint32_t kOutParts = 8;
 __global__ void __launch_bounds__(kBThreads) batch_out_kernel(const BatchTensor *tens, const CopyItem *items,
                                                               uint32_t B)
@@ -884,8 +899,8 @@ struct ptiB200Batch {
     std::vector<size_t> goff;  // Gram offset (doubles) of tensor b
     std::vector<size_t> loff;  // lambda offset (floats) of tensor b
     size_t elems = 0;
-    pti::DevBuf A, Ab, M, G, lam, norm2, ctrl, misc, plans, tens, tasks, copies;
-    uint32_t ntasks = 0;
+    pti::DevBuf A, Ab, M, G, W, acc, lam, norm2, ctrl, misc, plans, tens, tasks, copies;
+    uint32_t ntasks = 0, chunk_rows = pti::kMinChunkRows;
 };
 
 namespace pti {
@@ -905,6 +920,17 @@ int batch_build_plans(ptiB200Batch *bt, int sb)
         bt->hic[b].reset(h);
         for (uint32_t m = 0; m < 3; ++m) PTI_TRY(prepare_mode(h, m, s));
     }
+    // Chunks of the dense steps: about two and a half for each of the two CTAs
+    // of an SM.  Fewer leave SMs idle in a small batch, more pay for their
+    // fragments of W and their reductions: 20 tensors 0.209 / 0.176 / 0.155 ms
+    // an iteration with chunks of 512 / 256 / 128 rows, 128 tensors 0.828 /
+    // 0.871 / 0.990.
+    {
+        uint64_t rows = 0;
+        for (uint32_t d : bt->dims) rows += d;
+        bt->chunk_rows = kMinChunkRows;
+        while (bt->chunk_rows < 1024 && rows / 3 > (uint64_t)bt->chunk_rows * 5 * sm_count()) bt->chunk_rows *= 2;
+    }
     bt->sb = sb;
     std::vector<BatchPlan> hp(3 * (size_t)B);
     std::vector<uint32_t> ntiles(3 * (size_t)B);
@@ -917,27 +943,18 @@ int batch_build_plans(ptiB200Batch *bt, int sb)
             const HicooModePlan &P = h->hicoo_plan[m];
             BatchPlan p{};
             p.nnz = h->nnz;
-            p.nb = P.nb;
-            p.lblk = P.lblk.as<uint16_t>();
-            p.tile_block = P.tile_block.as<uint32_t>();
-            p.out_bind = P.binds[m].as<uint32_t>();
-            p.out_eind = P.einds[m].as<uint8_t>();
+            p.recs = P.recs.as<uint4>();
             for (uint32_t k = 0, i = 0; k < 3; ++k) {
                 if (k == m) continue;
-                p.in_bind[i] = P.binds[k].as<uint32_t>();
-                p.in_eind[i] = P.einds[k].as<uint8_t>();
-                p.in_dim[i] = bt->dims[3 * b + k];
                 p.A32[i] = A + bt->off[3 * b + k];
                 p.A16[i] = Ab + bt->off[3 * b + k];
                 ++i;
             }
-            p.vals = P.vals.as<float>();
             p.M = M + bt->off[3 * b + m];
             p.ntiles = P.ntiles;
-            p.sb = h->sb;
+            p.chunks = (bt->dims[3 * b + m] + bt->chunk_rows - 1) / bt->chunk_rows;
             p.R = bt->R[b];
             p.stride = bt->stride[b];
-            p.out_dim = bt->dims[3 * b + m];
             hp[3 * b + m] = p;
             ntiles[3 * b + m] = P.ntiles;
         }
@@ -946,27 +963,22 @@ int batch_build_plans(ptiB200Batch *bt, int sb)
     PTI_CUDA(cudaMemcpyAsync(bt->plans.ptr, hp.data(), hp.size() * sizeof(BatchPlan), cudaMemcpyHostToDevice, s),
              kMod);
 
-    // the queue: mode-0 tiles (largest tensors first), mode-0 dense steps
-    // (costliest first), mode-1 tiles (tensors whose dense step ends first
-    // first), ...
+    // the queue, each wave with the largest tensors first: a tensor whose step
+    // ends early starts its next mode early
     std::vector<uint32_t> order(B);
     std::vector<uint2> tasks;
-    auto dense_cost = [&](uint32_t b, uint32_t m) {
-        return (uint64_t)bt->dims[3 * b + m] * bt->R[b] * bt->R[b];
-    };
+    std::iota(order.begin(), order.end(), 0u);
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return bt->nnz[x] > bt->nnz[y]; });
     for (uint32_t m = 0; m < 3; ++m) {
-        std::iota(order.begin(), order.end(), 0u);
-        if (m == 0)
-            std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return bt->nnz[x] > bt->nnz[y]; });
-        else
-            std::stable_sort(order.begin(), order.end(),
-                             [&](uint32_t x, uint32_t y) { return dense_cost(x, m - 1) < dense_cost(y, m - 1); });
-        for (uint32_t b : order)
-            for (uint32_t t = 0; t < ntiles[3 * b + m]; ++t) tasks.push_back(make_uint2((3 * b + m) << 1, t));
-        std::iota(order.begin(), order.end(), 0u);
-        std::stable_sort(order.begin(), order.end(),
-                         [&](uint32_t x, uint32_t y) { return dense_cost(x, m) > dense_cost(y, m); });
-        for (uint32_t b : order) tasks.push_back(make_uint2(((3 * b + m) << 1) | 1u, 0u));
+        for (uint32_t b : order) {
+            const uint32_t pid = 3 * b + m;
+            tasks.push_back(make_uint2(pid << 2 | kInverse, 0u));
+            for (uint32_t t = 0; t < ntiles[pid]; ++t) tasks.push_back(make_uint2(pid << 2 | kTile, t));
+        }
+        for (uint32_t kind : {kSolve, kGram})
+            for (uint32_t b : order)
+                for (uint32_t c = 0; c < hp[3 * b + m].chunks; ++c)
+                    tasks.push_back(make_uint2((3 * b + m) << 2 | kind, c));
     }
     bt->ntasks = (uint32_t)tasks.size();
     PTI_CUDA(bt->tasks.alloc(padded(tasks.size() * sizeof(uint2)), s), kMod);
@@ -1009,7 +1021,8 @@ int batch_grid(const ptiB200Batch *bt, BatchKernel k, uint32_t *grid)
     return 0;
 }
 
-// Captures one iteration (counter reset, persistent kernel, iteration bump).
+// Captures one iteration (counter and accumulator reset, persistent kernel,
+// iteration bump).
 int batch_capture(ptiB200Batch *bt, const BatchArgs &a, BatchKernel k, cudaGraphExec_t *exec)
 {
     cudaStream_t s = bt->s;
@@ -1017,7 +1030,8 @@ int batch_capture(ptiB200Batch *bt, const BatchArgs &a, BatchKernel k, cudaGraph
     PTI_TRY(batch_grid(bt, k, &grid));
     cudaGraph_t graph = nullptr;
     PTI_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), kMod);
-    cudaMemsetAsync(bt->ctrl.ptr, 0, (1 + 4 * (size_t)bt->B) * 4, s);
+    cudaMemsetAsync(bt->ctrl.ptr, 0, ctrl_words(bt->B) * 4, s);
+    cudaMemsetAsync(bt->acc.ptr, 0, 3 * (size_t)bt->B * sizeof(BatchAcc), s);
     k<<<grid, kBThreads, kBatchSmem, s>>>(a);
     bump_kernel<<<1, 1, 0, s>>>(const_cast<uint32_t *>(a.iter));
     PTI_CUDA(cudaStreamEndCapture(s, &graph), kMod);
@@ -1041,6 +1055,8 @@ int batch_iterate(ptiB200Batch *bt, uint32_t niters, int mixed, uint32_t fp32_sw
     a.tasks = bt->tasks.as<uint2>();
     a.plans = bt->plans.as<BatchPlan>();
     a.tens = bt->tens.as<BatchTensor>();
+    a.acc = bt->acc.as<BatchAcc>();
+    a.W = bt->W.as<double>();
     a.ctrl = bt->ctrl.as<uint32_t>();
     a.iter = misc;
     a.fits = fits;
@@ -1050,6 +1066,7 @@ int batch_iterate(ptiB200Batch *bt, uint32_t niters, int mixed, uint32_t fp32_sw
     a.niters = niters;
     a.fp32_sweeps = fp32_sweeps;
     a.cpl = (uint32_t)cpl;
+    a.chunk_rows = bt->chunk_rows;
     a.mixed = mixed;
     a.wait_ns = kWaitNs;
     const uint32_t n16 = mixed && niters > fp32_sweeps ? niters - fp32_sweeps : 0, n32 = niters - n16;
@@ -1188,7 +1205,9 @@ int ptiB200BatchCreate(ptiB200Batch **out, ptiIndex ntensors, const ptiIndex *nd
     PTI_CUDA(bt->G.alloc(padded(gel * 8), s), kMod);
     PTI_CUDA(bt->lam.alloc(padded(lel * 4), s), kMod);
     PTI_CUDA(bt->norm2.alloc(padded((size_t)B * 8), s), kMod);
-    PTI_CUDA(bt->ctrl.alloc(padded((1 + 4 * (size_t)B) * 4), s), kMod);
+    PTI_CUDA(bt->W.alloc(padded(3 * (size_t)B * kRR * 8), s), kMod);
+    PTI_CUDA(bt->acc.alloc(padded(3 * (size_t)B * sizeof(BatchAcc)), s), kMod);
+    PTI_CUDA(bt->ctrl.alloc(padded(ctrl_words(B) * 4), s), kMod);
     PTI_CUDA(bt->misc.alloc(64, s), kMod);
     {
         std::vector<BatchTensor> ht(B);
@@ -1313,20 +1332,22 @@ int ptiB200BatchWaitProbe(ptiB200Batch *bt, double wait_seconds)
     PTI_CHECK(wait_seconds > 0.0 && wait_seconds <= 2.0, PTIERR_VALUE_ERROR, kMod,
               "wait bound must be in (0, 2] seconds");
     cudaStream_t s = bt->s;
-    // one task: the mode-1 dense step of tensor 0, which waits for the mode-0
-    // dense step -- a task this queue does not hold, so the counter it waits
+    // one task: the mode-1 inverse of tensor 0, which waits for the mode-0
+    // dense step -- tasks this queue does not hold, so the counter it waits
     // on stays 0 and the wait must give up after its bound
     DevBuf task;
     PTI_CUDA(task.alloc(64, s), kMod);
-    const uint2 t = make_uint2((1u << 1) | 1u, 0u);
+    const uint2 t = make_uint2(1u << 2 | kInverse, 0u);
     PTI_CUDA(cudaMemcpyAsync(task.ptr, &t, sizeof t, cudaMemcpyHostToDevice, s), kMod);
     uint32_t *misc = bt->misc.as<uint32_t>();
     PTI_CUDA(cudaMemsetAsync(misc, 0, 8, s), kMod);
-    PTI_CUDA(cudaMemsetAsync(bt->ctrl.ptr, 0, (1 + 4 * (size_t)bt->B) * 4, s), kMod);
+    PTI_CUDA(cudaMemsetAsync(bt->ctrl.ptr, 0, ctrl_words(bt->B) * 4, s), kMod);
     BatchArgs a{};
     a.tasks = task.as<uint2>();
     a.plans = bt->plans.as<BatchPlan>();
     a.tens = bt->tens.as<BatchTensor>();
+    a.acc = bt->acc.as<BatchAcc>();
+    a.W = bt->W.as<double>();
     a.ctrl = bt->ctrl.as<uint32_t>();
     a.iter = misc;
     a.fits = nullptr;
@@ -1335,6 +1356,7 @@ int ptiB200BatchWaitProbe(ptiB200Batch *bt, double wait_seconds)
     a.ntensors = bt->B;
     a.niters = 1;
     a.cpl = 4;
+    a.chunk_rows = bt->chunk_rows;
     a.wait_ns = (uint64_t)(wait_seconds * 1e9);
     uint32_t grid = 0;
     PTI_TRY(batch_grid(bt, batch_kernel(4, false), &grid));
