@@ -485,7 +485,7 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
     PTI_CUDA(cudaGetLastError(), mod);
     perm.reset();
 
-    // Blocks: bptr, binds.  Upper bound nb <= n until counted.
+    // Blocks: counted, then bptr and binds written at their exact sizes.
     DevBuf scan_tmp;
     PTI_CUDA(scan_tmp.alloc(padded(scan_tmp_elems<uint32_t>(n) * 4), s), mod);
     NewBlockFlag nbf{};
@@ -494,38 +494,34 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
     BlockOut bo{};
     bo.nmodes = N;
     bo.sb = sb;
-    DevBuf bptr_full;
-    std::array<DevBuf, kMaxModes> binds_full;
-    PTI_CUDA(bptr_full.alloc(padded((n + 1) * 8), s), mod);
-    for (uint32_t m = 0; m < N; ++m) {
-        nbf.sinds[m] = ex.sinds[m].as<uint32_t>();
-        bo.sinds[m] = ex.sinds[m].as<uint32_t>();
-        PTI_CUDA(binds_full[m].alloc(padded(n * 4), s), mod);
-        bo.binds[m] = binds_full[m].as<uint32_t>();
-    }
-    bo.bptr = bptr_full.as<uint64_t>();
+    const KeyChange kc{keys.as<uint64_t>(), N * sb};
     uint32_t nb32 = 0;
-    auto key_blocks = [&](auto n_modes) -> int {
-        constexpr int M = decltype(n_modes)::value;
-        KeyBlockOut<M> kb{ks, sb, keys.as<uint64_t>(), bptr_full.as<uint64_t>(), {}};
-        for (int m = 0; m < M; ++m) kb.binds[m] = binds_full[m].as<uint32_t>();
-        return exclusive_scan<uint32_t>(KeyChange{keys.as<uint64_t>(), N * sb}, kb, n, scan_tmp.as<uint32_t>(), &nb32, s);
-    };
-    if (!whole) PTI_TRY((exclusive_scan<uint32_t>(nbf, bo, n, scan_tmp.as<uint32_t>(), &nb32, s)));
-    else if (N == 3) PTI_TRY(key_blocks(std::integral_constant<int, 3>{}));
-    else PTI_TRY(key_blocks(std::integral_constant<int, 4>{}));
+    if (whole) {
+        PTI_TRY((scan_sums<uint32_t>(kc, n, scan_tmp.as<uint32_t>(), &nb32, s)));
+    } else {
+        for (uint32_t m = 0; m < N; ++m) nbf.sinds[m] = bo.sinds[m] = ex.sinds[m].as<uint32_t>();
+        PTI_TRY((scan_sums<uint32_t>(nbf, n, scan_tmp.as<uint32_t>(), &nb32, s)));
+    }
     const uint64_t nb = nb32;
     h->nb = nb;
-    PTI_CUDA(cudaMemcpyAsync(bptr_full.as<uint64_t>() + nb, &n, 8, cudaMemcpyHostToDevice, s), mod);
-    // shrink to exact sizes
     PTI_CUDA(h->bptr.alloc(padded((nb + 1) * 8), s), mod);
-    PTI_CUDA(cudaMemcpyAsync(h->bptr.ptr, bptr_full.ptr, (nb + 1) * 8, cudaMemcpyDeviceToDevice, s), mod);
-    for (uint32_t m = 0; m < N; ++m) {
-        PTI_CUDA(h->binds[m].alloc(padded(nb * 4), s), mod);
-        PTI_CUDA(cudaMemcpyAsync(h->binds[m].ptr, binds_full[m].ptr, nb * 4, cudaMemcpyDeviceToDevice, s), mod);
-        binds_full[m].reset();
+    for (uint32_t m = 0; m < N; ++m) PTI_CUDA(h->binds[m].alloc(padded(nb * 4), s), mod);
+    auto key_blocks = [&](auto n_modes) -> int {
+        constexpr int M = decltype(n_modes)::value;
+        KeyBlockOut<M> kb{ks, sb, keys.as<uint64_t>(), h->bptr.as<uint64_t>(), {}};
+        for (int m = 0; m < M; ++m) kb.binds[m] = h->binds[m].as<uint32_t>();
+        return scan_apply<uint32_t>(kc, kb, n, scan_tmp.as<uint32_t>(), s);
+    };
+    if (!whole) {
+        bo.bptr = h->bptr.as<uint64_t>();
+        for (uint32_t m = 0; m < N; ++m) bo.binds[m] = h->binds[m].as<uint32_t>();
+        PTI_TRY((scan_apply<uint32_t>(nbf, bo, n, scan_tmp.as<uint32_t>(), s)));
+    } else if (N == 3) {
+        PTI_TRY(key_blocks(std::integral_constant<int, 3>{}));
+    } else {
+        PTI_TRY(key_blocks(std::integral_constant<int, 4>{}));
     }
-    bptr_full.reset();
+    PTI_CUDA(cudaMemcpyAsync(h->bptr.as<uint64_t>() + nb, &n, 8, cudaMemcpyHostToDevice, s), mod);
 
     // Kernels: kptr over blocks.
     NewKernelFlag nkf{};
@@ -533,21 +529,17 @@ int convert_device(const ptiB200Tensor *coo, ptiB200Tensor *h, uint8_t sb, uint8
     nkf.sk = sk;
     nkf.bptr = h->bptr.as<uint64_t>();
     for (uint32_t m = 0; m < N; ++m) nkf.sinds[m] = ex.sinds[m].as<uint32_t>();
-    DevBuf kptr_full;
-    PTI_CUDA(kptr_full.alloc(padded((nb + 1) * 8), s), mod);
+    const KeyKernelFlag kkf{keys.as<uint64_t>(), h->bptr.as<uint64_t>(), N * sk};
     uint32_t nk32 = 0;
-    if (!whole)
-        PTI_TRY((exclusive_scan<uint32_t>(nkf, KernelOut{kptr_full.as<uint64_t>()}, nb, scan_tmp.as<uint32_t>(),
-                                          &nk32, s)));
-    else
-        PTI_TRY((exclusive_scan<uint32_t>(KeyKernelFlag{keys.as<uint64_t>(), h->bptr.as<uint64_t>(), N * sk},
-                                          KernelOut{kptr_full.as<uint64_t>()}, nb, scan_tmp.as<uint32_t>(), &nk32, s)));
+    if (!whole) PTI_TRY((scan_sums<uint32_t>(nkf, nb, scan_tmp.as<uint32_t>(), &nk32, s)));
+    else PTI_TRY((scan_sums<uint32_t>(kkf, nb, scan_tmp.as<uint32_t>(), &nk32, s)));
     const uint64_t nk = nk32;
     ex.nk = nk;
     PTI_CUDA(ex.kptr.alloc(padded((nk + 1) * 8), s), mod);
-    PTI_CUDA(cudaMemcpyAsync(ex.kptr.ptr, kptr_full.ptr, nk * 8, cudaMemcpyDeviceToDevice, s), mod);
+    const KernelOut ko{ex.kptr.as<uint64_t>()};
+    if (!whole) PTI_TRY((scan_apply<uint32_t>(nkf, ko, nb, scan_tmp.as<uint32_t>(), s)));
+    else PTI_TRY((scan_apply<uint32_t>(kkf, ko, nb, scan_tmp.as<uint32_t>(), s)));
     PTI_CUDA(cudaMemcpyAsync(ex.kptr.as<uint64_t>() + nk, &nb, 8, cudaMemcpyHostToDevice, s), mod);
-    kptr_full.reset();
 
     // Chunks.
     DevBuf ccount;

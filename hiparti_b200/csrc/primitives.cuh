@@ -95,25 +95,53 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(In in, uint64_
         }
 }
 
-// Exclusive scan: calls out(i, prefix_i, in(i)) for every i; returns the total
-// through *total_host (synchronous copy) if non-null.  `tmp` must hold
-// ceil(n / kScanTile) + 1 elements of T.
-template <class T, class In, class Out>
-int exclusive_scan(In in, Out out, uint64_t n, T *tmp, T *total_host, cudaStream_t s)
+// The two halves of an exclusive scan, for a caller that sizes its output by
+// the total: scan_sums returns the total through *total_host (synchronous copy)
+// if that is non-null; scan_apply then calls out(i, prefix_i, in(i)) for every
+// i.  `tmp` must hold ceil(n / kScanTile) + 1 elements of T.
+template <class T, class In>
+int scan_sums(In in, uint64_t n, T *tmp, T *total_host, cudaStream_t s)
 {
     const char *mod = "B200 scan";
-    uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
+    const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
     if (ntiles == 0) {
         if (total_host) *total_host = 0;
         return 0;
     }
     scan_reduce_kernel<T, In><<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, n, tmp);
     scan_tiles_kernel<T><<<1, 1024, 0, s>>>(tmp, ntiles);
-    scan_apply_kernel<T, In, Out><<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, n, tmp, out);
     PTI_CUDA(cudaGetLastError(), mod);
     if (total_host) {
         PTI_CUDA(cudaMemcpyAsync(total_host, tmp + ntiles, sizeof(T), cudaMemcpyDeviceToHost, s), mod);
         PTI_CUDA(cudaStreamSynchronize(s), mod);
+    }
+    return 0;
+}
+
+template <class T, class In, class Out>
+int scan_apply(In in, Out out, uint64_t n, const T *tmp, cudaStream_t s)
+{
+    const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
+    if (ntiles == 0) return 0;
+    scan_apply_kernel<T, In, Out><<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, n, tmp, out);
+    PTI_CUDA(cudaGetLastError(), "B200 scan");
+    return 0;
+}
+
+// Exclusive scan: calls out(i, prefix_i, in(i)) for every i; returns the total
+// through *total_host (synchronous copy) if non-null.
+template <class T, class In, class Out>
+int exclusive_scan(In in, Out out, uint64_t n, T *tmp, T *total_host, cudaStream_t s)
+{
+    PTI_TRY((scan_sums<T, In>(in, n, tmp, nullptr, s)));
+    PTI_TRY((scan_apply<T, In, Out>(in, out, n, tmp, s)));
+    if (total_host) {
+        *total_host = 0;
+        const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
+        if (ntiles) {
+            PTI_CUDA(cudaMemcpyAsync(total_host, tmp + ntiles, sizeof(T), cudaMemcpyDeviceToHost, s), "B200 scan");
+            PTI_CUDA(cudaStreamSynchronize(s), "B200 scan");
+        }
     }
     return 0;
 }

@@ -758,7 +758,7 @@ __global__ void pack_records_kernel(PackArgs pa, const uint32_t *perm, uint64_t 
 }
 
 // The schedule order of one tile of kHiTile nonzeros, by one CTA: the blocks
-// in their new order (bperm) with their nonzeros behind one another, then
+// in their new order with their nonzeros behind one another, then
 // stably by output row.  Writes for each position the nonzero there (order)
 // and its block, counted from the tile's first (lblk).
 //
@@ -766,15 +766,14 @@ __global__ void pack_records_kernel(PackArgs pa, const uint32_t *perm, uint64_t 
 // rows: a stable radix sort by 8-bit digits of the row, counted from the tile's
 // first, takes one pass for most tiles and at most four.  (A bitonic sort of
 // 64-bit {row, position} pairs, fed by passes that spelt out every nonzero's
-// block, took 0.63 ms a mode for 10M Zipf nonzeros; this takes 0.20.)
+// block, took 0.63 ms a mode for 10M Zipf nonzeros; this takes 0.12.)
 struct TileOrderArgs {
     uint64_t nnz, nb;
     uint32_t sb;
     const uint32_t *tile_block;
-    const uint64_t *nbptr;   // first nonzero of each block in the new order
-    const uint32_t *bperm;   // new order -> block
-    const uint32_t *out_bind;
-    const uint64_t *bptr;
+    const uint64_t *nbptr;     // first position of each block of the new order
+    const uint32_t *first;     // its first nonzero where it is stored
+    const uint32_t *out_bind;  // its output coordinate
     const uint8_t *out_eind;
     uint32_t *order;
     uint16_t *lblk;
@@ -807,18 +806,32 @@ __global__ void __launch_bounds__(kSortThreads) tile_order_kernel(TileOrderArgs 
 #pragma unroll
     for (uint32_t p = 0; p < PER; ++p) sum += s_key[1][tid * PER + p];
     uint32_t run = block_exclusive_scan<uint32_t>(sum, s_warp, total);
+    // the loads of all PER positions together; only the element offsets are
+    // read from where the nonzeros are stored
+    uint32_t z[PER], ob[PER], eo[PER];
 #pragma unroll
     for (uint32_t p = 0; p < PER; ++p) {
         const uint32_t pos = tid * PER + p;
         run += s_key[1][pos];
+        row[p] = run - 1;
+        z[p] = ob[p] = 0;
+        if (pos < cnt) {
+            const uint32_t j = b0 + row[p];
+            z[p] = __ldg(t.first + j) + (uint32_t)(z0 + pos - __ldg(t.nbptr + j));
+            ob[p] = __ldg(t.out_bind + j);
+        }
+    }
+#pragma unroll
+    for (uint32_t p = 0; p < PER; ++p) eo[p] = tid * PER + p < cnt ? __ldg(t.out_eind + z[p]) : 0u;
+#pragma unroll
+    for (uint32_t p = 0; p < PER; ++p) {
+        const uint32_t pos = tid * PER + p;
+        s_z[pos] = z[p];
+        s_l[pos] = (uint16_t)row[p];
+        // (a coordinate beyond 32 bits is out of range: behind every row)
+        const uint64_t o = ((uint64_t)ob[p] << t.sb) + eo[p];
         row[p] = 0xFFFFFFFFu;
         if (pos < cnt) {
-            const uint32_t i = run - 1, b = t.bperm[b0 + i];
-            const uint32_t z = (uint32_t)(t.bptr[b] + (z0 + pos - t.nbptr[b0 + i]));
-            s_z[pos] = z;
-            s_l[pos] = (uint16_t)i;
-            // (a coordinate beyond 32 bits is out of range: behind every row)
-            const uint64_t o = ((uint64_t)t.out_bind[b] << t.sb) + t.out_eind[z];
             row[p] = o < 0xFFFFFFFFull ? (uint32_t)o : 0xFFFFFFFFu;
             lo = min(lo, row[p]);
             hi = max(hi, row[p]);
@@ -900,7 +913,10 @@ __global__ void __launch_bounds__(256) plan_blocks_kernel(PlanGatherArgs g)
         uint32_t c[kMaxModes], q[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
         for (int k = 0; k < kMaxModes; ++k)
-            if (k < (int)g.nmodes) g.binds[k][j] = c[k] = g.binds_in[k][b];
+            if (k < (int)g.nmodes) {
+                if (k == (int)g.mode) c[k] = g.binds[k][j];  // in the new order already
+                else g.binds[k][j] = c[k] = g.binds_in[k][b];
+            }
         if (g.bquad) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) q[k == (int)g.mode ? 0 : k < (int)g.mode ? k + 1 : k] = c[k];
@@ -949,8 +965,9 @@ __global__ void __launch_bounds__(256) plan_nonzeros_kernel(PlanGatherArgs g)
     }
 }
 
-template <class T>
-__global__ void gather_kernel(const T *src, const uint32_t *perm, uint64_t n, T *dst)
+// (Bound by the random 32-byte sectors: four reads in flight a thread, from a
+// 16-byte load of perm, took 143 us instead of 134 for 20M values.)
+__global__ void gather_kernel(const float *src, const uint32_t *perm, uint64_t n, float *dst)
 {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         dst[i] = src[perm[i]];
@@ -966,14 +983,22 @@ __global__ void tile_block_kernel_t(const uint64_t *bptr, uint64_t nb, uint32_t 
     }
 }
 
-struct SizeIn {  // nonzeros of a block of the new order
-    const uint32_t *perm;
-    const uint64_t *bptr;
-    __device__ uint64_t operator()(uint64_t i) const
-    {
-        const uint32_t b = perm[i];
-        return bptr[b + 1] - bptr[b];
+// First nonzero and size of each block of the new order (nonzeros are indexed
+// by 32 bits).
+__global__ void __launch_bounds__(256) block_spans_kernel(const uint32_t *perm, uint64_t nb, const uint64_t *bptr,
+                                                          uint32_t *first, uint32_t *size)
+{
+    for (uint64_t j = (uint64_t)blockIdx.x * 256 + threadIdx.x; j < nb; j += (uint64_t)gridDim.x * 256) {
+        const uint32_t b = perm[j];
+        const uint64_t z = bptr[b];
+        first[j] = (uint32_t)z;
+        size[j] = (uint32_t)(bptr[b + 1] - z);
     }
+}
+
+struct SizeIn {
+    const uint32_t *p;
+    __device__ uint64_t operator()(uint64_t i) const { return p[i]; }
 };
 struct BptrOut {
     uint64_t *p;
@@ -1030,9 +1055,10 @@ static int build_plan(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arr
     const uint64_t nb = t->nb;
     PTI_CHECK(t->sb <= 8, PTIERR_VALUE_ERROR, mod, "sb_bits must be <= 8");
     // 1. blocks by output-mode block coordinate (stable)
-    DevBuf bkeys, bperm, nbptr, order;
+    DevBuf bperm, nbptr, first, order;  // (the sorted coordinates stay as P.binds[mode])
     {
         RadixScratchT<uint32_t> rs;
+        DevBuf &bkeys = P.binds[mode];
         PTI_CUDA(bkeys.alloc(padded(nb * 4), s), mod);
         PTI_CUDA(bperm.alloc(padded(nb * 4), s), mod);
         PTI_TRY(rs.alloc(nb, s));
@@ -1041,13 +1067,16 @@ static int build_plan(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arr
         const uint64_t brows = ((uint64_t)t->ndims[mode] + ((uint64_t)1 << t->sb) - 1) >> t->sb;
         PTI_TRY(radix_sort_pairs(bkeys, bperm, nb, (int)std::min(32u, bits_for_count(brows + 1)), rs, s));
     }
-    bkeys.reset();
     PTI_CUDA(nbptr.alloc(padded((nb + 1) * 8), s), mod);
+    PTI_CUDA(first.alloc(padded(nb * 4), s), mod);
     {
-        DevBuf tmp;
+        DevBuf tmp, bsize;
+        PTI_CUDA(bsize.alloc(padded(nb * 4), s), mod);
+        block_spans_kernel<<<grid_n(nb), 256, 0, s>>>(bperm.as<uint32_t>(), nb, t->bptr.as<uint64_t>(),
+                                                      first.as<uint32_t>(), bsize.as<uint32_t>());
         PTI_CUDA(tmp.alloc(padded(scan_tmp_elems<uint64_t>(nb) * 8), s), mod);
-        PTI_TRY((exclusive_scan<uint64_t>(SizeIn{bperm.as<uint32_t>(), t->bptr.as<uint64_t>()},
-                                          BptrOut{nbptr.as<uint64_t>()}, nb, tmp.as<uint64_t>(), nullptr, s)));
+        PTI_TRY((exclusive_scan<uint64_t>(SizeIn{bsize.as<uint32_t>()}, BptrOut{nbptr.as<uint64_t>()}, nb,
+                                          tmp.as<uint64_t>(), nullptr, s)));
         PTI_CUDA(cudaMemcpyAsync(nbptr.as<uint64_t>() + nb, tmp.as<uint64_t>() + (nb + kScanTile - 1) / kScanTile,
                                  8, cudaMemcpyDeviceToDevice, s), mod);
     }
@@ -1066,9 +1095,8 @@ static int build_plan(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arr
     ta.sb = t->sb;
     ta.tile_block = P.tile_block.as<uint32_t>();
     ta.nbptr = nbptr.as<uint64_t>();
-    ta.bperm = bperm.as<uint32_t>();
-    ta.out_bind = t->binds[mode].as<uint32_t>();
-    ta.bptr = t->bptr.as<uint64_t>();
+    ta.first = first.as<uint32_t>();
+    ta.out_bind = P.binds[mode].as<uint32_t>();
     ta.out_eind = t->einds[mode].as<uint8_t>();
     ta.order = order.as<uint32_t>();
     ta.lblk = P.lblk.as<uint16_t>();
@@ -1093,7 +1121,7 @@ static int build_plan(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arr
     g.lblk = P.lblk.as<uint16_t>();
     g.vals_in = t->vals.as<float>();
     for (uint32_t k = 0; k < N; ++k) {
-        PTI_CUDA(P.binds[k].alloc(padded(nb * 4), s), mod);
+        if (k != mode) PTI_CUDA(P.binds[k].alloc(padded(nb * 4), s), mod);
         PTI_CUDA(P.einds[k].alloc(padded(n), s), mod);
         g.dims[k] = t->ndims[k];
         g.binds_in[k] = t->binds[k].as<uint32_t>();
@@ -1388,8 +1416,8 @@ int mttkrp_scheduled(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t
         recs = P.recs.as<uint32_t>();
         if (vals_override) {  // substituted values, brought into record order
             if (!P.alt_vals.ptr) PTI_CUDA(P.alt_vals.alloc(padded(t->nnz * 4), s), mod);
-            gather_kernel<float><<<grid_n(t->nnz), 256, 0, s>>>(vals_override, P.perm.as<uint32_t>(), t->nnz,
-                                                                P.alt_vals.as<float>());
+            gather_kernel<<<grid_n(t->nnz), 256, 0, s>>>(vals_override, P.perm.as<uint32_t>(), t->nnz,
+                                                         P.alt_vals.as<float>());
             a.vals = P.alt_vals.as<float>();
         }
         for (uint32_t k = 0, i = 0; k < N; ++k)
