@@ -20,8 +20,9 @@ def _dims(N):
 def test_coo_panels_and_orders(lib, cuda, orc, N, R, dtype):
     import torch
     dims = _dims(N)
-    # the last tile holds one nonzero; from 16,384 nonzeros ranks above 128 take panels
-    nnz = 16385 if R > 128 else 4097 if R % 2 else 2049
+    # from where ranks above 128 take panels and orders above 4 schedules; the
+    # last tile holds one nonzero
+    nnz = 262_145 if N > 4 else 16_385
     inds, vals = synth.zipf_tensor(dims, nnz, s=1.1, seed=N * 1000 + R)
     mats = synth.factor_matrices(dims, R, seed=R + 1)
     dmats = [torch.from_numpy(m).to(cuda).to(getattr(torch, dtype)) for m in mats]
@@ -45,7 +46,7 @@ def test_first_use_under_capture_and_on_two_streams(lib, cuda, orc, N, R):
     the build."""
     import torch
     dims = _dims(N)
-    inds, vals = synth.uniform_tensor(dims, 20_000, seed=N)
+    inds, vals = synth.uniform_tensor(dims, 20_000 if N == 3 else 270_000, seed=N)
     mats = synth.factor_matrices(dims, R, seed=R)
     dmats = [torch.from_numpy(m).to(cuda) for m in mats]
     want = orc.mttkrp_coo_f64(inds, vals, mats, R, 1)[: dims[1]]
