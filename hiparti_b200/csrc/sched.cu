@@ -144,6 +144,30 @@ __device__ __forceinline__ void accumulate(float *acc, const RowPart<CPL, FT> (&
 
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;
 
+// Lane groups of G lanes, any G up to 32: 32 / G to a warp.  A warp's lanes
+// that make up no group take an index past the groups', where slices are empty.
+// Groups of 9, 10 and 6 lanes are used where rounding the lanes of a row up to a
+// power of two leaves room for fewer: 3 instead of 2 groups of a warp, or 5
+// instead of 4 (launch_r has the rule and what it measured).
+template <int G>
+struct Groups {
+    static constexpr uint32_t per_warp = 32 / G;
+    static constexpr uint32_t count = kSchedThreads / 32 * per_warp;
+    uint32_t g, lane;
+    __device__ __forceinline__ explicit Groups(uint32_t tid)
+    {
+        const uint32_t l = tid & 31;
+        if constexpr ((G & (G - 1)) == 0) {
+            g = tid / G;
+            lane = tid % G;
+        } else {
+            const bool idle = l >= per_warp * G;
+            g = idle ? kSchedThreads - 1 : (tid >> 5) * per_warp + l / G;
+            lane = idle ? 0u : l % G;
+        }
+    }
+};
+
 // Row runs of one thread group.  Products arrive in output-row order; a run
 // that ends is added into the output with one vector atomic per 4 columns,
 // except the runs a group shares with its neighbours in the CTA: the run that
@@ -152,7 +176,9 @@ constexpr uint32_t kNoRow = 0xFFFFFFFFu;
 // registers until merge(), where the group that started the row adds the
 // parked parts and writes the row once.  A row that fills many slices of a
 // tile (a hot row of a power-law mode) is so written once per tile instead of
-// once per group.
+// once per group.  (Writing it once per 8 groups shortens that chain and took
+// 2.27 instead of 2.31 ms on 50M Zipf nonzeros, but adds more FP32 parts in
+// global memory: 9.9e-7 instead of 5.7e-7 from FP64.)
 template <int CPL>
 struct RunWriter {
     float acc[CPL];
@@ -247,7 +273,7 @@ __device__ __forceinline__ void process_records(const uint32_t *s_rec, uint32_t 
                                                 float *s_slots, uint32_t *s_slot_row, uint8_t *s_slot_whole)
 {
     constexpr int RW = Rec<NIN>::words;
-    constexpr uint32_t kGroups = kSchedThreads / G;
+    constexpr uint32_t kGroups = Groups<G>::count;
     const uint32_t col = lane * CPL;
     const bool active = col < a.R;
     bool first_shared = false, last_shared = false;
@@ -329,7 +355,7 @@ __device__ __forceinline__ void walk_rows(const uint4 *s_rec, const float *s_v3,
                                           uint32_t j1, uint32_t g, uint32_t lane, const SchedArgs &a,
                                           float *s_slots, uint32_t *s_slot_row, uint8_t *s_slot_whole)
 {
-    constexpr uint32_t kGroups = kSchedThreads / G;
+    constexpr uint32_t kGroups = Groups<G>::count;
     const uint32_t col = lane * CPL;
     const bool active = col < a.R;
     bool first_shared = false, last_shared = false;
@@ -616,8 +642,9 @@ __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_sched_ker
     const uint4 *s_rec = reinterpret_cast<const uint4 *>(sm + L::rec);
     const float *s_v3 = reinterpret_cast<const float *>(sm + L::rval);
 
-    const uint32_t g = tid / G, lane = tid % G;
-    constexpr uint32_t kGroups = kSchedThreads / G;
+    const Groups<G> grp(tid);
+    const uint32_t g = grp.g, lane = grp.lane;
+    constexpr uint32_t kGroups = Groups<G>::count;
     // an odd slice length puts the groups' first records on different shared-memory banks
     const uint32_t per = ((n + kGroups - 1) / kGroups) | 1u;
     const uint32_t j0 = min(g * per, n), j1 = min(j0 + per, n);
@@ -676,8 +703,9 @@ __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kerne
         }
         return;
     }
-    const uint32_t g = tid / G, lane = tid % G;
-    constexpr uint32_t kGroups = kSchedThreads / G;
+    const Groups<G> grp(tid);
+    const uint32_t g = grp.g, lane = grp.lane;
+    constexpr uint32_t kGroups = Groups<G>::count;
     // an odd slice length puts the groups' first records on different shared-memory banks
     const uint32_t per = ((n + kGroups - 1) / kGroups) | 1u;
     const uint32_t j0 = min(g * per, n), j1 = min(j0 + per, n);
@@ -717,8 +745,9 @@ __global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArg
     __shared__ uint32_t s_slot_row[kSchedThreads];
     __shared__ uint8_t s_slot_whole[kSchedThreads];
     float *s_slots = reinterpret_cast<float *>(sm + (size_t)tile * RW * 4);  // [groups][G][CPL]
-    const uint32_t g = tid / G, lane = tid % G;
-    constexpr uint32_t kGroups = kSchedThreads / G;
+    const Groups<G> grp(tid);
+    const uint32_t g = grp.g, lane = grp.lane;
+    constexpr uint32_t kGroups = Groups<G>::count;
     const uint32_t per = ((n + kGroups - 1) / kGroups) | 1u;  // odd: groups start on different banks
     const uint32_t j0 = min(g * per, n), j1 = min(j0 + per, n);
     process_records<G, CPL, U, NIN, FT>(s_rec, n, j0, j1, g, lane, a, a.vals ? a.vals + z0 : nullptr, s_slots,
@@ -1256,7 +1285,7 @@ static int launch_hicoo(const SchedArgs &a0, unsigned ntiles, cudaStream_t s)
     if (cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rec_smem) != cudaSuccess)
         return PTIERR_CUDA_ERROR;
     static const uint64_t slots = cta_slots(kr, kSchedThreads, rec_smem);
-    a.part = part_len(kHiTile, split_for(ntiles, kHiTile, slots, kSchedThreads / G * U));
+    a.part = part_len(kHiTile, split_for(ntiles, kHiTile, slots, Groups<G>::count * U));
     const unsigned parts = (kHiTile + a.part - 1) / a.part;
     // whole tiles of 3-D FP32 runs are decoded in the kernel; parts of a tile
     // come from the records, which need no block table
@@ -1280,37 +1309,49 @@ static int launch_hicoo(const SchedArgs &a0, unsigned ntiles, cudaStream_t s)
 template <class FT, int NIN>
 static int launch_r(bool hicoo, bool wide, const SchedArgs &a, const uint32_t *recs, unsigned ntiles, cudaStream_t s)
 {
-    const uint32_t R = a.R;
-    if constexpr (sizeof(FT) == 2) {
-        if (wide) {
-            if (hicoo) {
-                if (R <= 8) return launch_hicoo<1, 8, FT, NIN>(a, ntiles, s);
-                if (R <= 16) return launch_hicoo<2, 8, FT, NIN>(a, ntiles, s);
-                if (R <= 32) return launch_hicoo<4, 8, FT, NIN>(a, ntiles, s);
-                if (R <= 64) return launch_hicoo<8, 8, FT, NIN>(a, ntiles, s);
-                return launch_hicoo<16, 8, FT, NIN>(a, ntiles, s);
+    // lanes a row takes, rounded up to the next group size
+    auto go = [&](auto lanes, auto cols) -> int {
+        constexpr int G = decltype(lanes)::value, CPL = decltype(cols)::value;
+        // records in flight per group of the COO walk
+        constexpr int U = CPL == 8 ? 2 : G <= 8 ? PTI_COO_U : G <= 16 ? PTI_COO_U64 : 2;
+        return hicoo ? launch_hicoo<G, CPL, FT, NIN>(a, ntiles, s) : launch_coo<G, CPL, U, FT, NIN>(a, recs, s);
+    };
+    auto pick = [&](auto cols) -> int {
+        constexpr int CPL = decltype(cols)::value;
+        const uint32_t q = (a.R + CPL - 1) / CPL;
+#define PTI_LANES(n) if (q <= n) return go(std::integral_constant<int, n>{}, cols)
+        PTI_LANES(1);
+        PTI_LANES(2);
+        PTI_LANES(4);
+        // 6, 9 and 10 lanes beside the powers of two, where that is faster (16 bytes a lane: FP32, wide BF16; 3- and 4-D).  All
+        // modes, power of two -> this: 9 and 10 lanes HiCOO 4-D 5M FP32 R = 40
+        // 997 -> 687 us, R = 36 995 -> 752; 3-D 8M Zipf R = 40 813 -> 667, BF16
+        // R = 80 861 -> 671; COO 3-D 5M Zipf R = 40 516 -> 421; but COO 4-D 3M
+        // BF16 R = 80 590 -> 634.  6 lanes COO 3-D 5M Zipf FP32 R = 24 341 ->
+        // 303, HiCOO 3-D 8M Zipf BF16 R = 48 527 -> 482; but HiCOO 3-D FP32
+        // R = 24 467 -> 477 and every 4-D one slower.  3 and 5 lanes lose more
+        // (walks of short rows are bound by their records) than they win.
+        if constexpr (CPL * sizeof(FT) == 16 && NIN == 2) {
+            if (!hicoo || sizeof(FT) == 2) {
+                if (q == 6) return go(std::integral_constant<int, 6>{}, cols);
             }
-            if (R <= 8) return launch_coo<1, 8, 2, FT, NIN>(a, recs, s);
-            if (R <= 16) return launch_coo<2, 8, 2, FT, NIN>(a, recs, s);
-            if (R <= 32) return launch_coo<4, 8, 2, FT, NIN>(a, recs, s);
-            if (R <= 64) return launch_coo<8, 8, 2, FT, NIN>(a, recs, s);
-            return launch_coo<16, 8, 2, FT, NIN>(a, recs, s);
         }
+        PTI_LANES(8);
+        if constexpr (CPL * sizeof(FT) == 16 && NIN >= 2) {
+            if (hicoo || NIN == 2 || sizeof(FT) == 4) {
+                PTI_LANES(9);
+                PTI_LANES(10);
+            }
+        }
+        PTI_LANES(16);
+        if constexpr (CPL == 4) return go(std::integral_constant<int, 32>{}, cols);
+        return PTIERR_VALUE_ERROR;  // not reached: R <= kPanel
+#undef PTI_LANES
+    };
+    if constexpr (sizeof(FT) == 2) {
+        if (wide) return pick(std::integral_constant<int, 8>{});
     }
-    if (hicoo) {
-        if (R <= 4) return launch_hicoo<1, 4, FT, NIN>(a, ntiles, s);
-        if (R <= 8) return launch_hicoo<2, 4, FT, NIN>(a, ntiles, s);
-        if (R <= 16) return launch_hicoo<4, 4, FT, NIN>(a, ntiles, s);
-        if (R <= 32) return launch_hicoo<8, 4, FT, NIN>(a, ntiles, s);
-        if (R <= 64) return launch_hicoo<16, 4, FT, NIN>(a, ntiles, s);
-        return launch_hicoo<32, 4, FT, NIN>(a, ntiles, s);
-    }
-    if (R <= 4) return launch_coo<1, 4, PTI_COO_U, FT, NIN>(a, recs, s);
-    if (R <= 8) return launch_coo<2, 4, PTI_COO_U, FT, NIN>(a, recs, s);
-    if (R <= 16) return launch_coo<4, 4, PTI_COO_U, FT, NIN>(a, recs, s);
-    if (R <= 32) return launch_coo<8, 4, PTI_COO_U, FT, NIN>(a, recs, s);
-    if (R <= 64) return launch_coo<16, 4, PTI_COO_U64, FT, NIN>(a, recs, s);
-    return launch_coo<32, 4, 2, FT, NIN>(a, recs, s);
+    return pick(std::integral_constant<int, 4>{});
 }
 
 // COO schedules of 5 to 8 modes: 4 columns per lane.
