@@ -89,13 +89,17 @@ __global__ void __launch_bounds__(256) kruskal_values_kernel(KVArgs a)
 // mode-0 row keep that factor row in registers, so a nonzero gathers the
 // other modes' rows only (2 instead of 3 for a 3-mode tensor).  Each value is
 // written to its input position (the schedule's permutation).
+//
+// A lane group takes four records at a time: their rows are in flight
+// together, and the group's four sums are reduced as one: each halving
+// exchanges the sums that the other half keeps, 5 shuffles for 16 lanes where
+// four separate sums take 16.  Three records and separate sums took 0.98 ms for
+// 20M nonzeros at R = 64 and 0.080 for 3M at R = 20; this takes 0.90 and 0.065.
+// (Values in schedule order and a scattering pass behind them: 0.86 ms for the
+// 20M, whose values and factors together pass the L2, but 0.50 instead of 0.49
+// for 12M and 0.33 instead of 0.28 for 8M.)
 constexpr uint32_t kKsTile = 2048;  // records per CTA at most (split_for)
-#ifndef PTI_KS_U
-#define PTI_KS_U 3
-#endif
-// records in flight per lane group: 3 (64 registers, 4 CTAs per SM) measured
-// a little faster than 2 (48 registers, 5 CTAs) on a 20M-nonzero tensor
-constexpr int kKsU = PTI_KS_U;
+constexpr int kKsU = 4;             // records in flight per lane group
 
 struct KSArgs {
     uint64_t nnz;
@@ -109,7 +113,7 @@ struct KSArgs {
 };
 
 template <int G, int NIN>
-__global__ void __launch_bounds__(256) kruskal_sched_kernel(KSArgs a)
+__global__ void __launch_bounds__(256, 4) kruskal_sched_kernel(KSArgs a)
 {
     static_assert(NIN == 1 || NIN == 2, "records of 4 words hold up to 3 modes");
     __shared__ __align__(128) uint4 s_rec[kKsTile];
@@ -141,62 +145,77 @@ __global__ void __launch_bounds__(256) kruskal_sched_kernel(KSArgs a)
     const uint32_t per = (n + kGroups - 1) / kGroups;
     const uint32_t j0 = min(g * per, n), j1 = min(j0 + per, n);
     const uint32_t col = lane * 4;
-    const bool active = col < a.R;
+    const bool active = col < a.R, tail = active && col + 4 > a.R;
     const uint32_t c0 = active ? col : 0u;  // inactive lanes read column 0 and are masked
     uint32_t cur = 0xFFFFFFFFu;
     float4 arow = make_float4(0.f, 0.f, 0.f, 0.f);
     for (uint32_t t = 0; t < per; t += kKsU) {
         uint4 r[kKsU];
-        bool valid[kKsU];
+        bool same = true;
 #pragma unroll
         for (int u = 0; u < kKsU; ++u) {
             const uint32_t j = j0 + t + u;
-            valid[u] = j < j1;
-            r[u] = valid[u] ? s_rec[j] : make_uint4(0u, 0u, 0u, 0u);
-        }
-        float4 f[kKsU][NIN];
-#pragma unroll
-        for (int u = 0; u < kKsU; ++u) {
-            const uint32_t rows[2] = {r[u].y, r[u].z};
-#pragma unroll
-            for (int k = 0; k < NIN; ++k) f[u][k] = load4(a.mats[1 + k] + (size_t)rows[k] * a.stride, c0);
-        }
-        // the mode-0 rows: the cached row while every record of the warp's
-        // batch continues it, else one gather per record
-        bool same = true;
-#pragma unroll
-        for (int u = 0; u < kKsU; ++u) same = same && (!valid[u] || r[u].x == cur);
-        float4 fa[kKsU];
-        if (__all_sync(0xffffffffu, same)) {
-#pragma unroll
-            for (int u = 0; u < kKsU; ++u) fa[u] = arow;
-        } else {
-#pragma unroll
-            for (int u = 0; u < kKsU; ++u) fa[u] = load4(a.mats[0] + (size_t)r[u].x * a.stride, c0);
-#pragma unroll
-            for (int u = 0; u < kKsU; ++u)
-                if (valid[u]) {
-                    cur = r[u].x;
-                    arow = fa[u];
-                }
+            // past the slice: any rows; no value is written
+            r[u] = j < j1 ? s_rec[j] : make_uint4(cur, 0u, 0u, 0u);
+            same = same && r[u].x == cur;
         }
         float s[kKsU];
+        auto sum = [&](float4 p) {
+            if (!active) p = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tail) p = mask4(p, col, a.R);
+            return (p.x + p.y) + (p.z + p.w);
+        };
+        auto rows = [&](int u, float4 (&f)[NIN]) {
+            const uint32_t row[2] = {r[u].y, r[u].z};
 #pragma unroll
-        for (int u = 0; u < kKsU; ++u) {
-            float4 p = fa[u];
+            for (int k = 0; k < NIN; ++k) f[k] = load4(a.mats[1 + k] + (size_t)row[k] * a.stride, c0);
+        };
+        auto product = [&](float4 p, const float4 (&f)[NIN]) {
 #pragma unroll
-            for (int k = 0; k < NIN; ++k) p = mul4(p, f[u][k]);
-            p = mask4(p, col, a.R);
-            s[u] = (p.x + p.y) + (p.z + p.w);
+            for (int k = 0; k < NIN; ++k) p = mul4(p, f[k]);
+            return p;
+        };
+        // the mode-0 row: the held one while every record of the warp's batch
+        // continues it, else one gather per record, two records at a time
+        if (__all_sync(0xffffffffu, same)) {
+            float4 f[kKsU][NIN];
+#pragma unroll
+            for (int u = 0; u < kKsU; ++u) rows(u, f[u]);
+#pragma unroll
+            for (int u = 0; u < kKsU; ++u) s[u] = sum(product(arow, f[u]));
+        } else {
+#pragma unroll
+            for (int h = 0; h < kKsU; h += 2) {
+                float4 f[2][NIN], fa[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    rows(h + u, f[u]);
+                    fa[u] = load4(a.mats[0] + (size_t)(r[h + u].x == 0xFFFFFFFFu ? 0u : r[h + u].x) * a.stride, c0);
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) s[h + u] = sum(product(fa[u], f[u]));
+                cur = r[h + 1].x;
+                arow = fa[1];
+            }
         }
+        if constexpr (G >= 4) {
+            // lane halves, then quarters, keep two and one of the four sums
+            const bool h = lane & (G / 2), q = lane & (G / 4);
+            const float k0 = (h ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, h ? s[0] : s[2], G / 2, G);
+            const float k1 = (h ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, h ? s[1] : s[3], G / 2, G);
+            float v = (q ? k1 : k0) + __shfl_xor_sync(0xffffffffu, q ? k0 : k1, G / 4, G);
 #pragma unroll
-        for (int u = 0; u < kKsU; ++u)
+            for (int o = G / 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
+            const uint32_t j = j0 + t + (h ? 2u : 0u) + (q ? 1u : 0u);
+            if (lane % (G / 4) == 0 && j < j1) a.out[__ldg(a.perm + z0 + j)] = v;
+        } else {
 #pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o, G);
-        if (lane == 0) {
+            for (int u = 0; u < kKsU; ++u) {
 #pragma unroll
-            for (int u = 0; u < kKsU; ++u)
-                if (valid[u]) a.out[__ldg(a.perm + z0 + j0 + t + u)] = s[u];
+                for (int o = G / 2; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o, G);
+                const uint32_t j = j0 + t + u;
+                if (lane == 0 && j < j1) a.out[__ldg(a.perm + z0 + j)] = s[u];
+            }
         }
     }
 }
