@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256) kruskal_values_kernel(KVArgs a)
 // (Values in schedule order and a scattering pass behind them: 0.86 ms for the
 // 20M, whose values and factors together pass the L2, but 0.50 instead of 0.49
 // for 12M and 0.33 instead of 0.28 for 8M.)
-constexpr uint32_t kKsTile = 2048;  // records per CTA at most (split_for)
+constexpr uint32_t kKsTile = 2048;  // records per CTA at most (tile_for)
 constexpr int kKsU = 4;             // records in flight per lane group
 
 struct KSArgs {
@@ -244,7 +244,7 @@ template <int G, int NIN>
 static int launch_ks_g(KSArgs a, cudaStream_t s)
 {
     static const uint64_t slots = cta_slots(kruskal_sched_kernel<G, NIN>, 256, 0);
-    a.tile = part_len(kKsTile, split_for((a.nnz + kKsTile - 1) / kKsTile, kKsTile, slots, 256 / G * kKsU));
+    a.tile = tile_for(a.nnz, kKsTile, slots, 256 / G * kKsU);
     kruskal_sched_kernel<G, NIN><<<(unsigned)((a.nnz + a.tile - 1) / a.tile), 256, 0, s>>>(a);
     return 0;
 }

@@ -1242,8 +1242,7 @@ static int launch_coo(const SchedArgs &a, const uint32_t *recs, cudaStream_t s)
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max) != cudaSuccess)
         return PTIERR_CUDA_ERROR;
     static const uint64_t slots = cta_slots(k, kSchedThreads, smem_max);
-    const uint32_t split = split_for((a.nnz + kTile - 1) / kTile, kTile, slots, kSchedThreads / G * UU);
-    const uint32_t tile = part_len(kTile, split);
+    const uint32_t tile = tile_for(a.nnz, kTile, slots, Groups<G>::count * 4);
     const size_t smem = (size_t)tile * RW * 4 + (size_t)kSchedThreads * CPL * 4;
     k<<<(unsigned)((a.nnz + tile - 1) / tile), kSchedThreads, smem, s>>>(a, recs, tile);
     return 0;

@@ -10,6 +10,24 @@ from hiparti_b200 import COOTensor, DeviceTensor, synth
 pytestmark = pytest.mark.gpu
 
 
+# a turn of the GPU is 592 tiles of 2048: within one, just over one, three even turns, more than five
+@pytest.mark.parametrize("nnz", [1_211_111, 1_212_417, 3_100_003, 6_100_001])
+@pytest.mark.parametrize("R", [16, 40])
+def test_even_turns(lib, cuda, orc, nnz, R):
+    import torch
+    dims = (300, 250, 200)
+    inds, vals = synth.uniform_tensor(dims, nnz, seed=nnz)
+    mats = synth.factor_matrices(dims, R, seed=R)
+    dmats = [torch.from_numpy(m).to(cuda) for m in mats]
+    eps = np.finfo(np.float32).eps
+    coo = DeviceTensor.from_coo(COOTensor(dims, inds, vals))
+    want = orc.mttkrp_coo_f64(inds, vals, mats, R, 1)[: dims[1]]
+    rows = np.bincount(inds[1], minlength=dims[1])[:, None]
+    got = coo.mttkrp(dmats, 1, rank=R).cpu().numpy()
+    assert np.all(np.abs(got - want) <= (3 + rows) * eps * want + 1e-30)
+    coo.free()
+
+
 @pytest.mark.parametrize("nnz", [1, 63, 257, 2047, 2049, 4099, 40_000])
 @pytest.mark.parametrize("R", [4, 10, 32, 128])
 @pytest.mark.parametrize("N", [3, 4])
