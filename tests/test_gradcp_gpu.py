@@ -120,3 +120,21 @@ def test_kruskal_values_every_group_shape(lib, cuda, N, R):
     want = model.sum(1)
     assert rel_err(got, want) < 1e-5
     dt.free()
+
+
+def test_loss_takes_the_shapes_of_a_difference(lib, cuda):
+    import torch
+    from hiparti_b200.autograd import cp_loss
+    dims = (30, 20, 10)
+    inds, vals = synth.uniform_tensor(dims, 500, seed=3)
+    dt = DeviceTensor.from_coo(COOTensor(dims, inds, vals))
+    facs = [torch.from_numpy(m).to(cuda) for m in synth.factor_matrices(dims, 8, seed=4)]
+    one = torch.tensor(0.25, device=cuda)
+    same = cp_loss(dt, one.expand(500).contiguous(), facs)
+    for v in (one, one.reshape(1)):
+        assert abs(float(cp_loss(dt, v, facs)) - float(same)) <= 1e-5 * float(same)
+    x = torch.from_numpy(vals).to(cuda)
+    for v in (x.reshape(1, -1), x.reshape(-1, 1), x[:-1]):
+        with pytest.raises(RuntimeError):
+            cp_loss(dt, v, facs)
+    dt.free()
