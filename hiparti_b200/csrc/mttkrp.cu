@@ -274,9 +274,15 @@ int mttkrp_device(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t R,
     if (t->nnz == 0) return 0;
     const int G = group_lanes(R);
     if (use_schedule(t, mode, R, stride, vals_override == nullptr, s)) {
-        PTI_TRY(prepare_mode(t, mode, s, arr));
-        if (arr && arr->all) PTI_CUDA(cudaStreamWaitEvent(s, arr->all, 0), mod);
-        return mttkrp_scheduled(t, mats, ft, R, stride, mats_order, mode, out, s, vals_override);
+        const int st = prepare_mode(t, mode, s, arr);
+        // where a schedule is only the faster way and there is no memory for
+        // it, the direct kernels still run: they need none
+        const bool direct = (N > 4 || R > 128) && st == PTIERR_CUDA_ERROR + (int)cudaErrorMemoryAllocation;
+        if (st && !direct) return st;
+        if (!direct) {
+            if (arr && arr->all) PTI_CUDA(cudaStreamWaitEvent(s, arr->all, 0), mod);
+            return mttkrp_scheduled(t, mats, ft, R, stride, mats_order, mode, out, s, vals_override);
+        }
     }
     if (arr && arr->all) PTI_CUDA(cudaStreamWaitEvent(s, arr->all, 0), mod);
 
@@ -870,8 +876,8 @@ int ptiB200MTTKRP(ptiB200Tensor *t, const void *const *dev_mats, int factor_type
 int ptiB200Prepare(ptiB200Tensor *t, ptiIndex mode, void *stream)
 {
     PTI_CHECK(t, PTIERR_VALUE_ERROR, "B200 Prepare", "null handle");
-    PTI_CHECK(t->nmodes <= 4 || t->nnz == 0, PTIERR_VALUE_ERROR, "B200 Prepare",
-              "schedules are prepared ahead for orders up to 4");
+    PTI_CHECK(t->hicoo || t->nmodes <= 4 || t->nnz == 0, PTIERR_VALUE_ERROR, "B200 Prepare",
+              "COO schedules are prepared ahead for orders up to 4");
     return pti::prepare_mode(t, mode, static_cast<cudaStream_t>(stream));
 }
 

@@ -1206,7 +1206,12 @@ int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals
         return 0;
     }
     PTI_TRY(ensure_err_word(t, s));
-    PTI_TRY(build_plan(t, mode, s, arr));
+    const int st = build_plan(t, mode, s, arr);
+    if (st) {  // what was allocated of it goes back
+        if (t->hicoo) t->hicoo_plan[mode] = HicooModePlan();
+        else t->coo_plan[mode] = CooModePlan();
+        return st;
+    }
     if (!capturing(s)) {
         if (!o.event) PTI_CUDA(cudaEventCreateWithFlags(&o.event, cudaEventDisableTiming), mod);
         PTI_CUDA(cudaEventRecord(o.event, s), mod);

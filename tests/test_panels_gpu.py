@@ -73,3 +73,27 @@ def test_first_use_under_capture_and_on_two_streams(lib, cuda, orc, N, R):
         assert np.abs(o.cpu().numpy() - want).max() <= 1e-5 * np.abs(want).max()
     dt.check()
     dt.free()
+
+
+def test_prepare_of_five_modes(lib, cuda, orc):
+    """HiCOO tensors of five modes have no schedule to build and say so by
+    succeeding; COO ones are refused."""
+    import torch
+    from hiparti_b200 import HiCOOTensor
+    dims, n = (4, 5, 6, 7, 8), 300
+    rng = np.random.default_rng(5)
+    inds = [rng.integers(0, d, n).astype(np.uint32) for d in dims]
+    vals = rng.random(n).astype(np.float32)
+    h = HiCOOTensor(dims, 4, 6, 8, [0, n], [[0]] * 5, inds, vals)
+    mats = synth.factor_matrices(dims, 8, seed=1)
+    dmats = [torch.from_numpy(m).to(cuda) for m in mats]
+    dt = DeviceTensor.from_hicoo(h)
+    dt.prepare()
+    want = orc.mttkrp_coo_f64(inds, vals, mats, 8, 2)[: dims[2]]
+    got = dt.mttkrp(dmats, 2, rank=8).cpu().numpy()
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+    dt.free()
+    dc = DeviceTensor.from_coo(COOTensor(dims, inds, vals))
+    with pytest.raises(Exception):
+        dc.prepare()
+    dc.free()
