@@ -57,7 +57,8 @@ struct SchedArgs {
     const uint8_t *in_eind[kMaxModes - 1];
     uint32_t in_dim[kMaxModes - 1];
     const void *in_mat[kMaxModes - 1];
-    const float *vals;
+    const float *vals;          // COO: substituted values, or null
+    const uint32_t *perm;       // COO: where each record's is among them; null: in record order
     float *out;
     uint32_t *err;
     const uint4 *bquad;         // HiCOO 4-D: per block {output, operand 0, 1, 2} block coordinates
@@ -269,8 +270,8 @@ __device__ __forceinline__ bool same_row_batch(const uint32_t (&orow)[U], uint32
 // in registers, one output row run at a time (RunWriter).
 template <int G, int CPL, int U, int NIN, class FT>
 __device__ __forceinline__ void process_records(const uint32_t *s_rec, uint32_t n, uint32_t j0, uint32_t j1,
-                                                uint32_t g, uint32_t lane, const SchedArgs &a, const float *alt,
-                                                float *s_slots, uint32_t *s_slot_row, uint8_t *s_slot_whole)
+                                                uint32_t g, uint32_t lane, const SchedArgs &a, float *s_slots,
+                                                uint32_t *s_slot_row, uint8_t *s_slot_whole)
 {
     constexpr int RW = Rec<NIN>::words;
     constexpr uint32_t kGroups = Groups<G>::count;
@@ -311,7 +312,7 @@ __device__ __forceinline__ void process_records(const uint32_t *s_rec, uint32_t 
                     wd[q] = r.x; wd[q + 1] = r.y; wd[q + 2] = r.z; wd[q + 3] = r.w;
                 }
                 orow[u] = wd[0];
-                val[u] = alt ? __ldg(alt + j + u) : __uint_as_float(wd[1 + NIN]);
+                val[u] = __uint_as_float(wd[1 + NIN]);
                 if (orow[u] != kNoRow && active) {
 #pragma unroll
                     for (int k = 0; k < NIN; ++k) f[u][k].load(base[k] + (size_t)wd[1 + k] * a.stride, 0);
@@ -713,7 +714,12 @@ __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kerne
 }
 
 // COO schedule: packed records sorted by output index; no sorting in the
-// kernel.  A CTA takes `tile` records (launch_coo sizes it).
+// kernel.  A CTA takes `tile` records (launch_coo sizes it).  Substituted values
+// (the residual of a CP gradient) are fetched while the records are on their
+// way and put into them, so the walk knows one kind of record: a load and a
+// choice per record less, every mode, COO 3M Zipf R = 64 281 -> 264 us, 1M R =
+// 16 51 -> 49.5, 4-D 5M R = 32 503 -> 489; 20M uniform R = 64 loss and gradient
+// 3.10 -> 3.03 ms, Zipf 2.92 -> 2.78.
 template <int G, int CPL, int U, int MINB, class FT, int NIN>
 __global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArgs a, const uint32_t *recs, uint32_t tile)
 {
@@ -734,6 +740,18 @@ __global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArg
         mbar_arrive_expect_tx(&mbar, bytes);
         bulk_g2s_ef(s_rec, recs + z0 * RW, bytes, &mbar);
     }
+    constexpr uint32_t kPer = (coo_tile(RW, CPL) + kSchedThreads - 1) / kSchedThreads;
+    float sub[kPer];
+    if (a.vals) {
+        uint32_t z[kPer];
+#pragma unroll
+        for (uint32_t i = 0; i < kPer; ++i) {
+            const uint32_t j = tid + i * kSchedThreads;
+            z[i] = j < n ? (a.perm ? __ldcs(a.perm + z0 + j) : (uint32_t)(z0 + j)) : 0;
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kPer; ++i) sub[i] = __ldcg(a.vals + z[i]);
+    }
     const bool ok = mbar_wait_bounded(&mbar, 0);
     if (!__syncthreads_and(ok)) {
         if (tid == 0) {
@@ -741,6 +759,14 @@ __global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArg
             mbar_wait_bounded(&mbar, 0);
         }
         return;
+    }
+    if (a.vals) {
+#pragma unroll
+        for (uint32_t i = 0; i < kPer; ++i) {
+            const uint32_t j = tid + i * kSchedThreads;
+            if (j < n) s_rec[(size_t)j * RW + 1 + NIN] = __float_as_uint(sub[i]);
+        }
+        __syncthreads();
     }
     __shared__ uint32_t s_slot_row[kSchedThreads];
     __shared__ uint8_t s_slot_whole[kSchedThreads];
@@ -750,8 +776,7 @@ __global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArg
     constexpr uint32_t kGroups = Groups<G>::count;
     const uint32_t per = ((n + kGroups - 1) / kGroups) | 1u;  // odd: groups start on different banks
     const uint32_t j0 = min(g * per, n), j1 = min(j0 + per, n);
-    process_records<G, CPL, U, NIN, FT>(s_rec, n, j0, j1, g, lane, a, a.vals ? a.vals + z0 : nullptr, s_slots,
-                                        s_slot_row, s_slot_whole);
+    process_records<G, CPL, U, NIN, FT>(s_rec, n, j0, j1, g, lane, a, s_slots, s_slot_row, s_slot_whole);
 }
 
 // ---------------------------------------------------------------------------
@@ -1464,7 +1489,20 @@ int mttkrp_scheduled(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t
         // records hold the operand modes in increasing order
         CooModePlan &P = t->coo_plan[mode];
         recs = P.recs.as<uint32_t>();
-        if (vals_override) {  // substituted values, brought into record order
+        // Substituted values are random reads through the permutation.  The walk
+        // does them beside its own copies where they and the factors share the
+        // L2; otherwise they would push the factor rows out of it, and a pass
+        // of their own brings them into record order first.  Loss and gradient,
+        // in the walk / in a pass, uniform: 8M R = 40 Zipf (45 MB) 0.97 / 1.02
+        // ms, 10M R = 64 (78 MB) 1.29 / 1.34, 18M R = 16 (91 MB) 1.32 / 1.31,
+        // 10M R = 64 (101 MB) 1.44 / 1.38, 14M R = 64 (133 MB) 2.25 / 2.00.
+        constexpr uint64_t kValsBesideFactors = 96'000'000;
+        uint64_t reused = t->nnz * 4;
+        for (uint32_t k = 0; k < N; ++k) reused += (uint64_t)t->ndims[k] * stride * (ft == PTI_B200_F32 ? 4 : 2);
+        if (vals_override && reused <= kValsBesideFactors) {
+            a.vals = vals_override;
+            a.perm = P.perm.as<uint32_t>();
+        } else if (vals_override) {
             if (!P.alt_vals.ptr) PTI_CUDA(P.alt_vals.alloc(padded(t->nnz * 4), s), mod);
             gather_kernel<<<grid_n(t->nnz), 256, 0, s>>>(vals_override, P.perm.as<uint32_t>(), t->nnz,
                                                          P.alt_vals.as<float>());
