@@ -27,7 +27,7 @@
 // for at I = 5,000 and R = 32 and which lie on every tensor's critical path
 // three times an iteration, so it is cut into row chunks for many SMs.  One CTA
 // a step, with tiles decoded by the CTA that walks them: 1.75 ms an iteration
-// of 128 tensors (10M nonzeros) and 0.99 of 20; this takes 0.81 and 0.16.
+// of 128 tensors (10M nonzeros) and 0.99 of 20; this takes 0.72 and 0.15.
 //
 // The queue is ordered in waves -- all mode-0 inverses and tiles, all mode-0
 // solves, all mode-0 Grams, all mode-1 inverses and tiles, ... -- and a task
@@ -443,6 +443,11 @@ __device__ void solve_task(const BatchTensor *__restrict__ gt, uint32_t m, uint3
     }
 }
 
+// v / d, given inv = 1 / d in FP64: rounded to FP32 once, from within 2^-51 of
+// the quotient, which is the rounded quotient unless it lies that close to the
+// middle of two FP32 numbers.
+__device__ __forceinline__ float scaled(float v, double inv) { return (float)((double)v * inv); }
+
 // A /= lambda, the BF16 copy and the Gram of one chunk's rows, and its slice of
 // the next mode's MTTKRP output zeroed (whose tiles wait for this step).  With
 // gram_bf16 (the iterations whose MTTKRPs gather BF16 factors) the Gram is
@@ -450,6 +455,9 @@ __device__ void solve_task(const BatchTensor *__restrict__ gt, uint32_t m, uint3
 // the next steps' right-hand sides and normal matrices come from the same
 // factors.  The warp's 8 scaled rows go through a shared-memory tile, each half
 // (4 rows) is one k-step for the tiles (p, q), p <= q, of the symmetric Gram.
+// A chunk of 462 rows (mean) took 23.8 us, 9 of them FP32 divisions by lambda
+// and 3 loads of M after the last mode; with scaled() and M fetched a block
+// ahead it takes 14, and an iteration of 128 tensors 0.72 ms instead of 0.81.
 __device__ void gram_task(const BatchTensor *__restrict__ gt, uint32_t b, uint32_t m, uint32_t chunk, uint32_t it,
                           const BatchArgs &a, BatchAcc *acc, unsigned char *sm, bool gram_bf16, double *s_red)
 {
@@ -467,16 +475,21 @@ __device__ void gram_task(const BatchTensor *__restrict__ gt, uint32_t b, uint32
                                        : fmaxf(__int_as_float(__ldcg(&acc->colmax[lane])), 1.f))
                             : 1.f;
     if (chunk == 0 && warp == 0 && colok) gt->lambda[lane] = lam;
+    const double inv_lam = 1.0 / (double)lam;
     double inner = 0.0;
     double *tile = reinterpret_cast<double *>(sm) + warp * (8 * kRowPad);
     double gacc[10][2];
 #pragma unroll
     for (int j = 0; j < 10; ++j) gacc[j][0] = gacc[j][1] = 0.0;
-    float next[8];  // the rows of the warp's next block
+    float next[8], nextm[8];  // the rows of A, and after the last mode of M, of the warp's next block
     auto fetch = [&](uint32_t row0) {
 #pragma unroll
         for (int q = 0; q < 8; ++q)
             next[q] = colok && row0 + q < r1 ? __ldcg(A + (size_t)(row0 + q) * stride + lane) : 0.f;
+        if (last)
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                nextm[q] = colok && row0 + q < r1 ? __ldcg(M + (size_t)(row0 + q) * stride + lane) : 0.f;
     };
     fetch(r0 + warp * 8);
     for (uint32_t row0 = r0 + warp * 8; row0 < r1; row0 += kWarps * 8) {
@@ -484,14 +497,14 @@ __device__ void gram_task(const BatchTensor *__restrict__ gt, uint32_t b, uint32
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             v[q] = next[q];
-            mm[q] = last && colok && row0 + q < r1 ? __ldcg(M + (size_t)(row0 + q) * stride + lane) : 0.f;
+            mm[q] = nextm[q];
         }
         fetch(row0 + kWarps * 8);
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const uint32_t row = row0 + q;
-            if (colok) v[q] = v[q] / lam;
+            if (colok) v[q] = scaled(v[q], inv_lam);
             const __nv_bfloat16 h = __float2bfloat16_rn(colok ? v[q] : 0.f);
             // the value the next MTTKRPs gather (and the fit's model uses)
             const double used = gram_bf16 ? (double)__bfloat162float(h) : (double)v[q];
@@ -653,7 +666,7 @@ __global__ void __launch_bounds__(kBThreads, 2) batch_als_kernel(BatchArgs a)
         // another takes the next one and, where that is settled, sees that it
         // may run.  Between the tasks, by one thread before the others went
         // on, this took 3.7 us of a tile's 9.9 (128 tensors: 0.85 ms an
-        // iteration; now 0.81).
+        // iteration; 0.81 so).
         if (tid == 32) publish();
         if (task.x == kNone) break;  // nothing follows the end of the queue: no copy is in flight
         const uint32_t pid = task.x >> 2, kind = task.x & 3u, b = pid / 3, m = pid % 3;
