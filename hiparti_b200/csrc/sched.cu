@@ -33,12 +33,11 @@
 namespace pti {
 
 
-// Nonzeros per CTA of the COO kernel at most.  Records of 8 words (4-D) with
-// FP32 rows take 1024, which fits a fourth CTA on an SM: 527 -> 507 us for the
-// four modes of a uniform 4-D tensor of 5M nonzeros at R = 32.  BF16 rows keep
-// 2048, as their walk feeds on the L1 that the fourth CTA's shared memory
-// would take (574 us, and 609 with 1024, for 5M Zipf nonzeros at R = 64).
-constexpr uint32_t coo_tile(int words, int cpl) { return cpl == 8 || words <= 4 ? 2048u : 8192u / words & ~3u; }
+// Nonzeros per CTA of the COO kernel: 2048, or what 32 KB hold of the records
+// of 8 modes.  (1024 of 8 words fit a fourth CTA on an SM, 505 -> 485 us for the
+// four modes of a uniform 4-D tensor of 5M nonzeros at R = 32, but add a hot
+// row's parts to the output twice as often, see coo_sched_kernel.)
+constexpr uint32_t coo_tile(int words) { return words <= 8 ? 2048u : 8192u / words & ~3u; }
 constexpr int kHiTile = kPlanTile; // nonzeros per CTA (HiCOO kernel)
 constexpr int kSchedThreads = 256;
 
@@ -61,10 +60,10 @@ struct SchedArgs {
     const uint32_t *perm;       // COO: where each record's is among them; null: in record order
     float *out;
     uint32_t *err;
+    bool cut;                   // COO: CTAs may take less than a tile
     const uint4 *bquad;         // HiCOO 4-D: per block {output, operand 0, 1, 2} block coordinates
     const uint4 *recs;          // HiCOO: decoded records of the schedule (HicooModePlan::recs)
     const float *rvals;         // HiCOO 4-D: their values
-    uint32_t part;              // hicoo_rec_kernel: nonzeros per CTA, at most kHiTile
 };
 
 
@@ -665,10 +664,6 @@ struct RecSmem {
 // schedule already holds decoded (HicooModePlan::recs, in output-row order
 // within the tile): one bulk copy stages them (and the 4-D values), then the
 // thread groups walk contiguous slices (walk_rows).
-//
-// With few tiles each is cut into parts of a.part records, one CTA each
-// (split_for; blockIdx.y is the part): a part is contiguous and in row order
-// like its tile.
 template <int G, int CPL, int U, class FT, int NIN>
 __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kernel(SchedArgs a)
 {
@@ -681,10 +676,8 @@ __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kerne
     float *s_v3 = reinterpret_cast<float *>(sm + L::rval);
     float *s_slots = reinterpret_cast<float *>(sm + L::slots);
     const uint32_t tid = threadIdx.x;
-    const uint32_t in_tile = blockIdx.y * a.part;  // < kHiTile: no part is empty in a full tile
-    const uint64_t z0 = (uint64_t)blockIdx.x * kHiTile + in_tile;
-    if (z0 >= a.nnz) return;
-    const uint32_t n = (uint32_t)min((uint64_t)min(a.part, kHiTile - in_tile), a.nnz - z0);
+    const uint64_t z0 = (uint64_t)blockIdx.x * kHiTile;
+    const uint32_t n = (uint32_t)min((uint64_t)kHiTile, a.nnz - z0);
     if (tid == 0) {
         mbar_init(&mbar, 1);
         mbar_fence_init();
@@ -714,7 +707,13 @@ __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kerne
 }
 
 // COO schedule: packed records sorted by output index; no sorting in the
-// kernel.  A CTA takes `tile` records (launch_coo sizes it).  Substituted values
+// kernel.  A CTA takes one tile, whatever their number: smaller ones are faster
+// where tiles are few (100,000 Zipf nonzeros in HiCOO 50 -> 25 us, COO 1M 55 ->
+// 49), but add the hot rows of a power-law mode to the output in more parts,
+// and the error of those sums against 64 bits grows (mean over ten tensors of
+// positive terms 8.6e-8 with whole tiles, 1.22e-7 with parts).  Calls whose other
+// choice is the direct kernel, which adds every product by itself, are cut
+// (a.cut; split.cuh): its error is 2e-4 where this has 3e-7.  Substituted values
 // (the residual of a CP gradient) are fetched while the records are on their
 // way and put into them, so the walk knows one kind of record: a load and a
 // choice per record less, every mode, COO 3M Zipf R = 64 281 -> 264 us, 1M R =
@@ -740,7 +739,7 @@ __global__ void __launch_bounds__(kSchedThreads, MINB) coo_sched_kernel(SchedArg
         mbar_arrive_expect_tx(&mbar, bytes);
         bulk_g2s_ef(s_rec, recs + z0 * RW, bytes, &mbar);
     }
-    constexpr uint32_t kPer = (coo_tile(RW, CPL) + kSchedThreads - 1) / kSchedThreads;
+    constexpr uint32_t kPer = (coo_tile(RW) + kSchedThreads - 1) / kSchedThreads;
     float sub[kPer];
     if (a.vals) {
         uint32_t z[kPer];
@@ -1264,15 +1263,18 @@ int prepare_mode(ptiB200Tensor *t, uint32_t mode, cudaStream_t s, const Arrivals
 template <int G, int CPL, int U, class FT, int NIN>
 static int launch_coo(const SchedArgs &a, const uint32_t *recs, cudaStream_t s)
 {
-    constexpr uint32_t RW = Rec<NIN>::words, kTile = coo_tile(RW, CPL);
+    constexpr uint32_t RW = Rec<NIN>::words, kTile = coo_tile(RW);
     constexpr size_t smem_max = (size_t)kTile * RW * 4 + (size_t)kSchedThreads * CPL * 4;
     // more operands hold more registers per nonzero in flight
     constexpr int UU = NIN > 4 ? 1 : (NIN >= 3 && U > 2 ? 2 : U);
     auto k = coo_sched_kernel<G, CPL, UU, PTI_COO_MINB, FT, NIN>;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max) != cudaSuccess)
         return PTIERR_CUDA_ERROR;
-    static const uint64_t slots = cta_slots(k, kSchedThreads, smem_max);
-    const uint32_t tile = tile_for(a.nnz, kTile, slots, Groups<G>::count * 4);
+    uint32_t tile = kTile;
+    if (a.cut) {
+        static const uint64_t slots = cta_slots(k, kSchedThreads, smem_max);
+        tile = tile_for(a.nnz, kTile, slots, Groups<G>::count * 4);
+    }
     const size_t smem = (size_t)tile * RW * 4 + (size_t)kSchedThreads * CPL * 4;
     k<<<(unsigned)((a.nnz + tile - 1) / tile), kSchedThreads, smem, s>>>(a, recs, tile);
     return 0;
@@ -1299,10 +1301,17 @@ constexpr bool use_records()
 }
 
 template <int G, int CPL, class FT, int NIN>
-static int launch_hicoo(const SchedArgs &a0, unsigned ntiles, cudaStream_t s)
+static int launch_hicoo(const SchedArgs &a, unsigned ntiles, cudaStream_t s)
 {
     constexpr int U = NIN == 3 || CPL == 8 ? 2 : PTI_HICOO_U;  // nonzeros in flight per group
-    SchedArgs a = a0;
+    if constexpr (!use_records<FT, NIN>()) {
+        constexpr size_t smem = HiSmem<NIN, CPL>::total;
+        auto k = hicoo_sched_kernel<G, CPL, U, FT, NIN>;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            return PTIERR_CUDA_ERROR;
+        k<<<ntiles, kSchedThreads, smem, s>>>(a);
+        return 0;
+    }
     auto kr = hicoo_rec_kernel<G, CPL, U, FT, NIN>;
     size_t rec_smem = RecSmem<NIN, CPL>::total;
     if (sizeof(FT) == 2 && PTI_REC_BF16_CTAS > 0) {
@@ -1313,22 +1322,7 @@ static int launch_hicoo(const SchedArgs &a0, unsigned ntiles, cudaStream_t s)
     }
     if (cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rec_smem) != cudaSuccess)
         return PTIERR_CUDA_ERROR;
-    static const uint64_t slots = cta_slots(kr, kSchedThreads, rec_smem);
-    a.part = part_len(kHiTile, split_for(ntiles, kHiTile, slots, Groups<G>::count * U));
-    const unsigned parts = (kHiTile + a.part - 1) / a.part;
-    // whole tiles of 3-D FP32 runs are decoded in the kernel; parts of a tile
-    // come from the records, which need no block table
-    if constexpr (!use_records<FT, NIN>()) {
-        if (parts == 1) {
-            constexpr size_t smem = HiSmem<NIN, CPL>::total;
-            auto k = hicoo_sched_kernel<G, CPL, U, FT, NIN>;
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-                return PTIERR_CUDA_ERROR;
-            k<<<ntiles, kSchedThreads, smem, s>>>(a);
-            return 0;
-        }
-    }
-    kr<<<dim3(ntiles, parts), kSchedThreads, rec_smem, s>>>(a);
+    kr<<<ntiles, kSchedThreads, rec_smem, s>>>(a);
     return 0;
 }
 
@@ -1458,6 +1452,7 @@ int mttkrp_scheduled(ptiB200Tensor *t, const void *const *mats, int ft, uint32_t
     a.out_dim = t->ndims[mode];
     a.out = out;
     a.err = err_word(t);
+    a.cut = N > 4 || R > kPanel;
     const uint32_t *recs = nullptr;
     unsigned ntiles = 0;
     if (t->hicoo) {

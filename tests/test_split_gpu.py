@@ -1,4 +1,4 @@
-"""GPU: schedule tiles cut into parts for tensors of few tiles.  Sizes around
+"""GPU: tensors of few tiles, and the CP model's tiles cut for them.  Sizes around
 one tile, a part and a wave, with rows that continue across parts; MTTKRP and
 the CP model against FP64 (all terms positive: the FP32 summation bound of an
 element is (modes + nonzeros of its row) * eps times the element)."""
@@ -25,6 +25,9 @@ def test_even_turns(lib, cuda, orc, nnz, R):
     rows = np.bincount(inds[1], minlength=dims[1])[:, None]
     got = coo.mttkrp(dmats, 1, rank=R).cpu().numpy()
     assert np.all(np.abs(got - want) <= (3 + rows) * eps * want + 1e-30)
+    model = coo.kruskal_values(dmats, rank=R).cpu().numpy()
+    p = mats[0][inds[0][::97], :R].astype(np.float64) * mats[1][inds[1][::97], :R] * mats[2][inds[2][::97], :R]
+    assert np.all(np.abs(model[::97] - p.sum(1)) <= (3 + R) * eps * p.sum(1))
     coo.free()
 
 
