@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(kSchedThreads, PTI_HICOO_MINB) hicoo_rec_kerne
 // (a.cut; split.cuh): its error is 2e-4 where this has 3e-7.  Substituted values
 // (the residual of a CP gradient) are fetched while the records are on their
 // way and put into them, so the walk knows one kind of record: a load and a
-// choice per record less, every mode, COO 3M Zipf R = 64 281 -> 264 us, 1M R =
+// choice per record less, every mode and both sides cut into even turns, COO 3M Zipf R = 64 281 -> 264 us, 1M R =
 // 16 51 -> 49.5, 4-D 5M R = 32 503 -> 489; 20M uniform R = 64 loss and gradient
 // 3.10 -> 3.03 ms, Zipf 2.92 -> 2.78.
 template <int G, int CPL, int U, int MINB, class FT, int NIN>
